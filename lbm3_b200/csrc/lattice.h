@@ -39,15 +39,22 @@ LBM_HD constexpr int cx(int d) { return packed(d) % 3 - 1; }
 LBM_HD constexpr int cy(int d) { return (packed(d) / 3) % 3 - 1; }
 LBM_HD constexpr int cz(int d) { return packed(d) / 9 - 1; }
 
-// Direction with velocity (x, y, z), each in {-1, 0, 1}.
+// Direction with velocity (x, y, z), each in {-1, 0, 1}: the inverse of
+// packed().  A switch like packed(), not a search over it: the compiler folds
+// thousands of these in every unrolled kernel.
 LBM_HD constexpr int dirOf(int x, int y, int z) {
-    const int key = (x + 1) + 3 * (y + 1) + 9 * (z + 1);
-    int r = 0;
-    for (int d = 0; d < Q; ++d)
-        if (packed(d) == key) r = d;
-    return r;
+    switch ((x + 1) + 3 * (y + 1) + 9 * (z + 1)) {
+        case 0: return 25; case 1: return 18; case 2: return 23; case 3: return 10;
+        case 4: return 3;  case 5: return 7;  case 6: return 19; case 7: return 13;
+        case 8: return 22; case 9: return 11; case 10: return 5; case 11: return 16;
+        case 12: return 2; case 13: return 0; case 14: return 1; case 15: return 15;
+        case 16: return 6; case 17: return 12; case 18: return 21; case 19: return 14;
+        case 20: return 20; case 21: return 8; case 22: return 4; case 23: return 9;
+        case 24: return 24; case 25: return 17; default: return 26;
+    }
 }
 
+// inv() flips the velocity: key 26 - k.
 LBM_HD constexpr int inv(int d) { return dirOf(-cx(d), -cy(d), -cz(d)); }
 
 LBM_HD constexpr float weight(int d) {
