@@ -180,7 +180,7 @@ unsigned long long levelBytes(const lbm::HostLevel& H, int storage) {
     b += bytes(H.rowI.size(), sizeof(int)) * 6;                     // compressed rows
     b += bytes(H.perIndex.size(), sizeof(int)) * 2;                 // periodic index, source
     b += bytes(H.segCell.size(), sizeof(int4)) + bytes(H.segLen.size(), sizeof(int));  // bulk segments
-    b += bytes(H.specialCells.size(), sizeof(int)) + bytes(H.rotorCells.size(), sizeof(int));
+    b += bytes(H.specialCells.size(), sizeof(int4)) + bytes(H.rotorCells.size(), sizeof(int));
     for (const auto& R : H.rotors)
         b += bytes(R.rotorMap.size(), sizeof(int)) + bytes(R.interpolation.size(), sizeof(unsigned)) +
              bytes(R.index.size(), sizeof(int)) + bytes(3 * 27 * R.index.size(), sizeof(float));
@@ -787,7 +787,12 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
                 d.seg = own(upload(seg, s));
                 d.segLen = own(upload(H.segLen, s));
                 d.segCount = static_cast<int>(seg.size());
-                d.special = own(upload(H.specialCells, s));
+                std::vector<int4> special(H.specialCells.size());
+                for (size_t q = 0; q < special.size(); ++q) {
+                    const int cell = H.specialCells[q], kp = H.kPlus[cell];
+                    special[q] = make_int4(cell, H.jPlus[cell], kp, H.jPlus[kp]);
+                }
+                d.special = own(upload(special, s));
                 d.specialCount = static_cast<int>(H.specialCells.size());
                 d.rotorCells = own(upload(H.rotorCells, s));
                 d.rotorCellCount = static_cast<int>(H.rotorCells.size());
@@ -1043,8 +1048,7 @@ int lbm_batch_create(lbm_grids* const* grids, int count, lbm_batch** out) {
         for (int q = 0; q < count; ++q) {
             const lbm::DevLevel& d = b->members[q]->levels[0].dev;
             levels.push_back(d);
-            const int items = d.segCount + (d.specialCount + 127) / 128;
-            itemStart.push_back(itemStart.back() + items);
+            itemStart.push_back(itemStart.back() + lbm::pairItems(d));
             for (int i = 0; i < d.obChunkCount; ++i) open.push_back(make_int2(q, i));
             perStart.push_back(perStart.back() + d.perCount);
             cells += d.cellCount;

@@ -592,97 +592,148 @@ __global__ void __launch_bounds__(kTile, LBM3_TMA_MIN_BLOCKS) collideBulkTma(Dev
     }
 }
 
+// Per-thread columns in shared memory of the listed-cell update: the
+// pre-collision populations and the packed link codes of a wall-adjacent cell.
+template <class T, int N> struct SpecialScratch {
+    T pre[26][N];
+    unsigned code[7][N];
+};
+
 // Cells outside the bulk segments, one thread per listed cell: wall-adjacent
 // fluid cells get the interpolated bounceback of Zhao & Yong (2017) with a
 // moving-wall term and momentum-exchange force
 // (applyIBB, include/boundaryConditions/interpolatedBouncebackFunctions.h:43-157,
 // and the write loop of include/updateGrid.h:143-176); the rest (cells whose
 // +1 neighbour wraps) collide and stream like bulk cells.
-template <bool F, class S, bool kRotors = false>
-__device__ __forceinline__ void collideSpecialCell(const DevLevel& g, int cell) {
+//
+// A few thousand cells: bound by the length of one thread's chain of loads.
+// Everything a wall-adjacent cell needs is therefore loaded before the
+// collision, together with the populations; the pre-collision values and the
+// link codes wait in shared memory (lane-private columns, so no barrier), and a link's
+// position in the packed codes is the population count of the lower links.
+// (Read per link from global memory instead, each linked direction was a
+// divergent branch with one or two dependent loads: a collide-stream launch of
+// a three-level sphere, 2,984 wall-adjacent cells on the finest of 59,000 to
+// 160,000 cells, took 28 us on average and takes 13.6; a 150x46x58 channel with
+// a body 39 and 20.)
+template <bool F, class S, bool kRotors, int N>
+__device__ __forceinline__ void collideSpecialCell(const DevLevel& g, int cell, const int (&nb)[8],
+                                                   const int* ijk, SpecialScratch<Real<S>, N>& sc, int t) {
     const int wm = __ldg(g.wallMap + cell);
-    int nb[8], ijk[3];
-    decodeNbr(g, cell, nb, kRotors ? ijk : nullptr);
     using T = Real<S>;
     T f[27];
     readPre<F, S>(g, nb, f);
+    const int nw = g.wallCount;
+    unsigned wallData = 0u;
+    T uwx = T(0), uwy = T(0), uwz = T(0);
+    double force[3] = {0.0, 0.0, 0.0};
+    if (wm >= 0) {
+        wallData = __ldg(g.wallData + wm);
+        uwx = __ldg(g.wallVel + wm);
+        uwy = __ldg(g.wallVel + nw + wm);
+        uwz = __ldg(g.wallVel + 2 * nw + wm);
+        if (g.useIBB) {
+#pragma unroll
+            for (int q = 0; q < 7; ++q) sc.code[q][t] = __ldg(g.linkLength + q * nw + wm);
+        }
+        if (g.trackWallForce) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) force[q] = g.wallForce[q * nw + wm];
+        }
+#pragma unroll
+        for (int d = 1; d < 27; ++d) sc.pre[d - 1][t] = f[d];
+    }
     T gx = g.gx, gy = g.gy, gz = g.gz, lambda = collConsts<T>(g).lambda;
-    if (kRotors) cellRotorForcing<F, S>(g, ijk, wm, f, gx, gy, gz, lambda);
+    if constexpr (kRotors) {
+        const int at[3] = {ijk[0], ijk[1], ijk[2]};
+        cellRotorForcing<F, S>(g, at, wm, f, gx, gy, gz, lambda);
+    }
     collideCumulantT(f, collConsts<T>(g), lambda, gx, gy, gz);
     const Dither D = stepDither<F, S>(g, kSaltCollide);
     if (wm < 0) {
         writePost<F, S>(g, nb, f, D);
         return;
     }
-    const unsigned wallData = __ldg(g.wallData + wm);
-    const int nw = g.wallCount;
-    const T uwx = __ldg(g.wallVel + wm), uwy = __ldg(g.wallVel + nw + wm), uwz = __ldg(g.wallVel + 2 * nw + wm);
     T dRho, ux, uy, uz;
     macroFromF(f, dRho, ux, uy, uz);
-    T out[27];
-#pragma unroll
-    for (int d = 0; d < 27; ++d) out[d] = f[d];
     T fx = T(0), fy = T(0), fz = T(0);
-    int link = 0;
-    unsigned code = 0u;
-    const S* base = static_cast<const S*>(g.f);
-#pragma unroll
-    for (int d = 1; d < 27; ++d) {
-        if (!((wallData >> d) & 1u)) continue;
-        const int id = inv(d);
-        const T eu = T(cx(id)) * uwx + T(cy(id)) * uwy + T(cz(id)) * uwz;
-        const T wallTerm = T(6) * weightT<T>(id) * (T(1) + dRho) * eu;
-        T gamma = T(0.5);
-        if (g.useIBB) {
-            if ((link & 3) == 0) code = __ldg(g.linkLength + (link >> 2) * nw + wm);
-            const unsigned c8 = (code >> (8 * (link & 3))) & 255u;
-            const T q = static_cast<T>(c8) / T(254);
-            gamma = q < T(0.01f) ? T(0.01f) : q > T(1) ? T(1) : q;
-            ++link;
-        }
-        // pre-collision value of direction d, still unchanged in memory
-        const T fPre = Store<S>::ld(base + (long long)preSlot<F>(d) * g.stride + nb[preNbr(d)]);
-        const T invDen = T(1) / (T(1) + gamma);
-        const T r = ((T(1) - gamma) * invDen) * fPre + (gamma * invDen) * f[id] + (gamma * invDen) * f[d] +
-                    invDen * wallTerm;
-        fx += -f[d] * (T(cx(d)) - uwx) + r * (T(cx(id)) - uwx);
-        fy += -f[d] * (T(cy(d)) - uwy) + r * (T(cy(id)) - uwy);
-        fz += -f[d] * (T(cz(d)) - uwz) + r * (T(cz(id)) - uwz);
-        out[d] = r;
-    }
-    // writes: a linked direction goes to the next pre-collision slot of its
-    // inverse (inside the wall cell), the others stream as usual
+    // a linked direction goes to the next pre-collision slot of its inverse
+    // (inside the wall cell), the others stream as usual
     S* wbase = static_cast<S*>(g.f);
+    const long long stride = g.stride;
     const unsigned cb = D.cell(cell);
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
-        const bool linked = d != 0 && ((wallData >> d) & 1u);
-        const int slot = linked ? (F ? inv(d) : d) : postSlot<F>(d);
-        stD(wbase + (long long)slot * g.stride + nb[postNbr(d)], out[d], D, cb, d);
+        T v = f[d];
+        int slot = postSlot<F>(d);
+        if (d != 0 && ((wallData >> d) & 1u)) {
+            const int id = inv(d);
+            const T eu = T(cx(id)) * uwx + T(cy(id)) * uwy + T(cz(id)) * uwz;
+            const T wallTerm = T(6) * weightT<T>(id) * (T(1) + dRho) * eu;
+            T gamma = T(0.5);
+            if (g.useIBB) {
+                const int link = __popc(wallData & ((1u << d) - 2u));
+                const unsigned c8 = (sc.code[link >> 2][t] >> (8 * (link & 3))) & 255u;
+                const T q = static_cast<T>(c8) / T(254);
+                gamma = q < T(0.01f) ? T(0.01f) : q > T(1) ? T(1) : q;
+            }
+            const T fPre = sc.pre[d > 0 ? d - 1 : 0][t];
+            const T invDen = T(1) / (T(1) + gamma);
+            v = ((T(1) - gamma) * invDen) * fPre + (gamma * invDen) * f[id] + (gamma * invDen) * f[d] +
+                invDen * wallTerm;
+            fx += -f[d] * (T(cx(d)) - uwx) + v * (T(cx(id)) - uwx);
+            fy += -f[d] * (T(cy(d)) - uwy) + v * (T(cy(id)) - uwy);
+            fz += -f[d] * (T(cz(d)) - uwz) + v * (T(cz(id)) - uwz);
+            slot = F ? inv(d) : d;
+        }
+        stD(wbase + (long long)slot * stride + nb[postNbr(d)], v, D, cb, d);
     }
     if (g.trackWallForce && !(wallData & 1u)) {
-        g.wallForce[wm] += double(fx);
-        g.wallForce[nw + wm] += double(fy);
-        g.wallForce[2 * nw + wm] += double(fz);
+        g.wallForce[wm] = force[0] + double(fx);
+        g.wallForce[nw + wm] = force[1] + double(fy);
+        g.wallForce[2 * nw + wm] = force[2] + double(fz);
     }
 }
 
-template <bool F, class S>
-__global__ void __launch_bounds__(kBlock) collideList(DevLevel g) {
-    advanceDither<F, S>(g);
-    const int idx = blockIdx.x * kBlock + threadIdx.x;
+// One entry {cell, jPlus, kPlus, jkPlus} of the special list.
+template <bool F, class S, int N>
+__device__ __forceinline__ void collideListed(const DevLevel& g, int idx, SpecialScratch<Real<S>, N>& sc, int t) {
     if (idx >= g.specialCount) return;
-    collideSpecialCell<F, S>(g, __ldg(g.special + idx));
+    const int4 rows = __ldg(g.special + idx);
+    int nb[8];
+    rowNbr(g, rows, nb);
+    collideSpecialCell<F, S, false, N>(g, rows.x, nb, nullptr, sc, t);
+}
+
+// The same as a call, for the packed kernel: inlined there, the listed cells'
+// registers made its tile loop spill (104 against 101 us for eight 64^3
+// domains in FP16).
+template <bool F, class S, int N>
+__device__ __noinline__ void collideListedCall(const DevLevel& g, int idx, SpecialScratch<Real<S>, N>& sc, int t) {
+    collideListed<F, S, N>(g, idx, sc, t);
+}
+
+constexpr int kListBlock = 64;
+
+template <bool F, class S>
+__global__ void __launch_bounds__(kListBlock) collideList(DevLevel g) {
+    __shared__ SpecialScratch<Real<S>, kListBlock> sc;
+    advanceDither<F, S>(g);
+    collideListed<F, S>(g, blockIdx.x * kListBlock + threadIdx.x, sc, threadIdx.x);
 }
 
 // Cells a rotor can reach while it turns, one thread each: special-cell
 // update with the rotor forcing before the collision.
 template <bool F, class S>
-__global__ void __launch_bounds__(kBlock) collideRotorList(DevLevel g) {
+__global__ void __launch_bounds__(kListBlock) collideRotorList(DevLevel g) {
+    __shared__ SpecialScratch<Real<S>, kListBlock> sc;
     advanceDither<F, S>(g);
-    const int idx = blockIdx.x * kBlock + threadIdx.x;
+    const int idx = blockIdx.x * kListBlock + threadIdx.x;
     if (idx >= g.rotorCellCount) return;
-    collideSpecialCell<F, S, true>(g, __ldg(g.rotorCells + idx));
+    const int cell = __ldg(g.rotorCells + idx);
+    int nb[8], ijk[3];
+    decodeNbr(g, cell, nb, ijk);
+    collideSpecialCell<F, S, true, kListBlock>(g, cell, nb, ijk, sc, threadIdx.x);
 }
 
 // Work items of one launch: special chunks [0, S) first (kTile listed cells
@@ -694,6 +745,7 @@ __global__ void __launch_bounds__(kBlock) collideRotorList(DevLevel g) {
 template <bool F, class S>
 __global__ void __launch_bounds__(kTile, LBM3_PREFETCH_MIN_BLOCKS) collidePrefetch(DevLevel g) {
     __shared__ int slot[2];
+    __shared__ SpecialScratch<Real<S>, kTile> sc;
     const int nSpecial = (g.specialCount + kTile - 1) / kTile;
     const int t = threadIdx.x;
     int parity = 0;
@@ -708,8 +760,7 @@ __global__ void __launch_bounds__(kTile, LBM3_PREFETCH_MIN_BLOCKS) collidePrefet
     };
     int item = fetch();
     while (item < nSpecial) {
-        const int q = item * kTile + t;
-        if (q < g.specialCount) collideSpecialCell<F, S>(g, __ldg(g.special + q));
+        collideListed<F, S>(g, item * kTile + t, sc, t);
         item = fetch();
     }
     int4 dCur, dNext;
@@ -764,6 +815,7 @@ __global__ void __launch_bounds__(kTile, LBM3_PREFETCH_MIN_BLOCKS) collidePrefet
 // LBM3_PAIR_PREFETCH the next tile's populations are also loaded into
 // registers during the current tile's collision.
 constexpr int kHalf = kTile / 2;
+static_assert(kHalf == kListedPerItem, "a work item of the paired kernels holds one listed cell per thread");
 
 #ifndef LBM3_PAIR_MIN_BLOCKS
 #define LBM3_PAIR_MIN_BLOCKS 8
@@ -840,29 +892,31 @@ __device__ __forceinline__ void loadTilePair(const DevLevel& g, const int4& d, i
 template <bool F, class S>
 __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePair(DevLevel g) {
     __shared__ int slot[2];
-    const int nSpecial = (g.specialCount + kTile - 1) / kTile;
+    __shared__ SpecialScratch<float, kHalf> sc;
+    const int nSpecial = (g.specialCount + kHalf - 1) / kHalf;
     const int t = threadIdx.x;
     int parity = 0;
     advanceDither<F, S>(g);
     const Dither D = stepDither<F, S>(g, kSaltCollide);
+    // a CTA's first two items are its own (blockIdx and blockIdx + gridDim), so
+    // the first tile's loads wait for no atomic; the counter hands out the rest
+    const int G = gridDim.x;
     auto fetch = [&]() {
-        if (t == 0) slot[parity] = atomicAdd(g.work, 1);
+        if (t == 0) slot[parity] = 2 * G + atomicAdd(g.work, 1);
         __syncthreads();
         const int v = slot[parity];
         parity ^= 1;
         return v;
     };
-    int item = fetch();
-    while (item < nSpecial) {
-        const int q = item * kTile + t;
-        if (q < g.specialCount) collideSpecialCell<F, S>(g, __ldg(g.special + q));
-        if (q + kHalf < g.specialCount) collideSpecialCell<F, S>(g, __ldg(g.special + q + kHalf));
-        item = fetch();
+    int item = blockIdx.x, next = item + G;
+    while (item < nSpecial) {  // CTA-uniform
+        collideListed<F, S>(g, item * kHalf + t, sc, t);
+        item = next;
+        next = fetch();
     }
     int4 dCur;
     int lCur;
     loadDesc(g, item - nSpecial, dCur, lCur);
-    int next = fetch();
 #if LBM3_PAIR_PREFETCH
     Pair fn[27];
     loadTilePair<F, S>(g, dCur, t, lCur, fn);
@@ -1256,16 +1310,8 @@ __device__ __forceinline__ void openLoad(const DevLevel& g, int idx, unsigned un
     c.uNormalRef = g.obUnRef[idx];
     c.target = __ldg(g.obTarget + idx);
     c.beta = __ldg(g.obBeta + idx);
-    const int n = g.cellCount;
     int nb[8];
-    nb[0] = c.rows.x;
-    nb[1] = c.rows.x + 1 < n ? c.rows.x + 1 : 0;
-    nb[2] = c.rows.y;
-    nb[3] = c.rows.y + 1 < n ? c.rows.y + 1 : 0;
-    nb[4] = c.rows.z;
-    nb[5] = c.rows.z + 1 < n ? c.rows.z + 1 : 0;
-    nb[6] = c.rows.w;
-    nb[7] = c.rows.w + 1 < n ? c.rows.w + 1 : 0;
+    rowNbr(g, c.rows, nb);
     const S* base = static_cast<const S*>(g.f);
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
@@ -1639,6 +1685,7 @@ template <bool F, class S>
 __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePacked(DevBatch b) {
     __shared__ int slot[2];
     __shared__ DevLevel sg;
+    __shared__ SpecialScratch<float, kHalf> sc;
     const int t = threadIdx.x;
     if constexpr (sizeof(S) == 2) {
         // every domain's next step seed (advanceDither of the single-domain launch)
@@ -1649,8 +1696,11 @@ __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePacked(Dev
             }
     }
     int parity = 0;
+    const int D = b.domainCount;
+    // the counter of a domain hands out the items after the first ones of its
+    // home CTAs, which are theirs without an atomic
     auto fetch = [&](int domain) {
-        if (t == 0) slot[parity] = atomicAdd(b.work + domain, 1);
+        if (t == 0) slot[parity] = (int(gridDim.x) - domain + D - 1) / D + atomicAdd(b.work + domain, 1);
         __syncthreads();
         const int v = slot[parity];
         parity ^= 1;
@@ -1659,24 +1709,21 @@ __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePacked(Dev
     // Each domain has its own item counter.  A CTA starts on its home domain
     // (blockIdx modulo the domain count) and moves on to the next domain when
     // that one runs out, so it stages a descriptor at most once per domain.
-    const int D = b.domainCount;
     int dom = static_cast<int>(blockIdx.x % unsigned(D));
     for (int visited = 0; visited < D; ++visited, dom = dom + 1 == D ? 0 : dom + 1) {
         const int count = b.itemStart ? __ldg(b.itemStart + dom + 1) - __ldg(b.itemStart + dom) : b.collideCount;
         if (count <= 0) continue;
-        int item = fetch(dom);
+        int item = visited == 0 ? int(blockIdx.x) / D : fetch(dom);
         if (item >= count) continue;  // CTA-uniform
         __syncthreads();              // every thread is done with the previous descriptor
         stageLevel(b.levels + dom, sg);
         __syncthreads();
-        const int nSpecial = (sg.specialCount + kTile - 1) / kTile;
+        const int nSpecial = (sg.specialCount + kHalf - 1) / kHalf;
         while (item < count) {  // CTA-uniform: items come through shared memory
             int next;
             if (item < nSpecial) {  // CTA-uniform branch: both sides fetch once
                 next = fetch(dom);
-                const int q = item * kTile + t;
-                if (q < sg.specialCount) collideSpecialCell<F, S>(sg, __ldg(sg.special + q));
-                if (q + kHalf < sg.specialCount) collideSpecialCell<F, S>(sg, __ldg(sg.special + q + kHalf));
+                collideListedCall<F, S>(sg, item * kHalf + t, sc, t);
             } else {
                 int4 d;
                 int l;
@@ -1766,7 +1813,7 @@ template <class K> int persistentGrid(K kernel, int block, int smem) {
 template <bool F, class S> struct RunCollidePair {
     static void run(const DevLevel& g, cudaStream_t s) {
         if constexpr (!std::is_same<S, double>::value) {
-            const int items = g.segCount + (g.specialCount + kTile - 1) / kTile;
+            const int items = pairItems(g);
             if (items > 0) {
                 DevBatch b{};
                 b.levels = g.self;
@@ -1777,7 +1824,7 @@ template <bool F, class S> struct RunCollidePair {
                 const int grid = persistentGrid(collidePacked<F, S>, kHalf, 0);
                 collidePacked<F, S><<<std::min(grid, items), kHalf, 0, s>>>(b);
             }
-            if (g.rotorCellCount > 0) collideRotorList<F, S><<<blocksFor(g.rotorCellCount), kBlock, 0, s>>>(g);
+            if (g.rotorCellCount > 0) collideRotorList<F, S><<<(g.rotorCellCount + kListBlock - 1) / kListBlock, kListBlock, 0, s>>>(g);
         }
     }
 };
@@ -1809,7 +1856,7 @@ template <bool F, class S> struct RunCollideOther {
             // the paired kernel with the descriptor as a kernel parameter
             // (faster on one large domain than the packed kernel's staged copy)
             if constexpr (!std::is_same<S, double>::value) {
-                const int items = g.segCount + (g.specialCount + kTile - 1) / kTile;
+                const int items = pairItems(g);
                 if (items > 0) {
                     const int grid = persistentGrid(collidePair<F, S>, kHalf, 0);
                     collidePair<F, S><<<std::min(grid, items), kHalf, 0, s>>>(g);
@@ -1821,7 +1868,7 @@ template <bool F, class S> struct RunCollideOther {
                 persistentGrid(collideBulkTma<!F, S>, kTile, tmaSmemBytes<S>());
                 collideBulkTma<F, S><<<std::min(grid, g.segCount), kTile, tmaSmemBytes<S>(), s>>>(g);
             }
-            if (g.specialCount > 0) collideList<F, S><<<blocksFor(g.specialCount), kBlock, 0, s>>>(g);
+            if (g.specialCount > 0) collideList<F, S><<<(g.specialCount + kListBlock - 1) / kListBlock, kListBlock, 0, s>>>(g);
         } else {
             // bulk segments and listed cells in one persistent launch
             const int items = g.segCount + (g.specialCount + kTile - 1) / kTile;
@@ -1830,7 +1877,7 @@ template <bool F, class S> struct RunCollideOther {
                 collidePrefetch<F, S><<<std::min(grid, items), kTile, 0, s>>>(g);
             }
         }
-        if (g.rotorCellCount > 0) collideRotorList<F, S><<<blocksFor(g.rotorCellCount), kBlock, 0, s>>>(g);
+        if (g.rotorCellCount > 0) collideRotorList<F, S><<<(g.rotorCellCount + kListBlock - 1) / kListBlock, kListBlock, 0, s>>>(g);
     }
 };
 

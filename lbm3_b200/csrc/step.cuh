@@ -14,7 +14,8 @@ namespace lbm {
 
 // open-boundary cells per CTA of the boundary kernel
 constexpr int kOpenChunk = 128;
-
+// listed (wall-adjacent) cells per work item of the paired kernels
+constexpr int kListedPerItem = 64;
 
 // One forcing rotor as the collide kernels see it (RotorViewStruct,
 // include/types.h:217-219), with this step's angle as cosine and sine.
@@ -52,8 +53,9 @@ struct DevLevel {
     const int4* seg;
     const int* segLen;
     int segCount;
-    // cells collided outside the bulk segments (wall-adjacent)
-    const int* special;
+    // cells collided outside the bulk segments (wall-adjacent):
+    // {cell, jPlus, kPlus, jkPlus}
+    const int4* special;
     int specialCount;
     int* errorFlag;          // set to nonzero when a bounded device wait gives up
     int* work;               // [2] work-item counter and finished-CTA count of the
@@ -150,6 +152,11 @@ struct DevInterface {
     double omegaCoarse, omegaFine;  // 1 / (3 nu + 1/2) of each level
 };
 
+// Work items of a level in the paired kernels: listed cells, then bulk tiles.
+inline int pairItems(const DevLevel& g) {
+    return g.segCount + (g.specialCount + kListedPerItem - 1) / kListedPerItem;
+}
+
 // Collision constants in the arithmetic type T.
 template <class T> __device__ __forceinline__ const CollisionConstsT<T>& collConsts(const DevLevel& g);
 template <> __device__ __forceinline__ const CollisionConstsT<float>& collConsts<float>(const DevLevel& g) {
@@ -190,6 +197,19 @@ __device__ __forceinline__ void decodeNbr(const DevLevel& g, int cell, int (&nb)
         ijk[1] = __ldg(g.rowJ + row);
         ijk[2] = __ldg(g.rowK + row);
     }
+}
+
+// The same neighbours from a stored record {cell, jPlus, kPlus, jkPlus}.
+__device__ __forceinline__ void rowNbr(const DevLevel& g, const int4& rows, int (&nb)[8]) {
+    const int n = g.cellCount;
+    nb[0] = rows.x;
+    nb[1] = rows.x + 1 < n ? rows.x + 1 : 0;
+    nb[2] = rows.y;
+    nb[3] = rows.y + 1 < n ? rows.y + 1 : 0;
+    nb[4] = rows.z;
+    nb[5] = rows.z + 1 < n ? rows.z + 1 : 0;
+    nb[6] = rows.w;
+    nb[7] = rows.w + 1 < n ? rows.w + 1 : 0;
 }
 
 // Typed population storage.  Half and bfloat16 hold the shifted value
