@@ -383,8 +383,9 @@ typedef struct lbm_batch_info {
     long long cells;          /* sum of the members' cells (ghosts included) */
     int collide_items;        /* collide-stream work items of all members     */
     int open_chunks;          /* open-boundary CTAs per step                  */
-    int periodic_cells;       /* periodic ghost cells per step                */
-    int launches_per_step;    /* kernels one packed step launches (<= 3)      */
+    int periodic_cells;       /* periodic ghost cells of all members          */
+    int launches_per_step;    /* kernels one packed step launches: up to 3, and
+                                 one per 16 members that are periodic boxes   */
 } lbm_batch_info;
 int lbm_batch_create(lbm_grids* const* grids, int count, lbm_batch** out);
 int lbm_batch_update(lbm_batch* b, int coarse_steps);

@@ -81,6 +81,10 @@ long long planeStride(long long n, int storage) {
 struct LevelState {
     lbm::Info info;
     int iterationsSinceTrackerReset = 0;
+    // wrapped levels (DevLevel::wrapped): the ghosts hold their sources' values,
+    // so the next step may be a wrapped one; a wrapped step has run since the
+    // ghosts were last refreshed
+    bool ghostsCurrent = false, flushPending = false;
     int rowCount = 0;
     int wallCellCount = 0;
     int wallAdjacentCount = 0;
@@ -179,6 +183,7 @@ unsigned long long levelBytes(const lbm::HostLevel& H, int storage) {
     b += bytes(n, sizeof(int)) * 2;                                 // shifter, wallMap
     b += bytes(H.rowI.size(), sizeof(int)) * 6;                     // compressed rows
     b += bytes(H.perIndex.size(), sizeof(int)) * 2;                 // periodic index, source
+    b += bytes(H.wrapSkip.size(), sizeof(unsigned));                // cells the ghost-free step leaves out
     b += bytes(H.segCell.size(), sizeof(int4)) + bytes(H.segLen.size(), sizeof(int));  // bulk segments
     b += bytes(H.specialCells.size(), sizeof(int4)) + bytes(H.rotorCells.size(), sizeof(int));
     for (const auto& R : H.rotors)
@@ -254,24 +259,65 @@ void advanceRotors(LevelState& L) {
 void updateSingleGrid(lbm_grids* g, LevelState& L, cudaStream_t stream) {
     if (!L.rotors.empty()) advanceRotors(L);
     const bool flip = L.info.esotwistFlipper;
-    if (g->timingKernels) {
-        const size_t k = static_cast<size_t>(g->kernelEventsUsed);
-        ck(cudaEventRecord(g->kernelEvents[k], stream), "event");
-        lbm::launchCollideStream(L.dev, flip, stream);
-        ck(cudaEventRecord(g->kernelEvents[k + 1], stream), "event");
-        g->kernelEventsUsed += 2;
+    const bool wrapped = L.dev.wrapped && L.ghostsCurrent;
+    const size_t k = static_cast<size_t>(g->kernelEventsUsed);
+    if (g->timingKernels) ck(cudaEventRecord(g->kernelEvents[k], stream), "event");
+    if (wrapped) {
+        const lbm::DevLevel* level = &L.dev;
+        lbm::launchWrapped(&level, 1, flip, stream);
+        lbm::launchRotorCells(L.dev, flip, stream);
     } else {
         lbm::launchCollideStream(L.dev, flip, stream);
     }
+    if (g->timingKernels) {
+        ck(cudaEventRecord(g->kernelEvents[k + 1], stream), "event");
+        g->kernelEventsUsed += 2;
+    }
     L.info.esotwistFlipper = !flip;  // applyStreaming
     lbm::launchOpenBoundary(L.dev, L.info.esotwistFlipper, stream);
-    lbm::launchPeriodic(L.dev, L.info.esotwistFlipper, stream);
+    if (wrapped) L.flushPending = true;
+    else lbm::launchPeriodic(L.dev, L.info.esotwistFlipper, stream);
+    L.ghostsCurrent = true;
     L.info.iterationsFinished++;
     L.iterationsSinceTrackerReset++;
 }
 
+// The end of a series of steps: the ordinary state (ghosts refreshed) of a
+// wrapped level, on the stream its last step ran on.
+void finishSteps(LevelState& L, cudaStream_t stream) {
+    if (!L.flushPending) return;
+    lbm::launchWrappedFlush(L.dev, L.info.esotwistFlipper, stream);
+    L.flushPending = false;
+}
+void finishSteps(lbm_grids* g) {
+    for (LevelState& L : g->levels) finishSteps(L, g->stream);
+}
+
+// A wrapped level whose ghosts do not repeat their sources yet (a new state
+// that a program or an initial condition set) steps once with ghost copies.
+bool needsGhostStep(const lbm_grids* g) {
+    return g->levels[0].dev.wrapped && !g->levels[0].ghostsCurrent;
+}
+
+// After the populations were set from outside: see whether the ghosts repeat
+// their sources.  The stream is idle afterwards.
+void checkGhosts(lbm_grids* g) {
+    LevelState& L = g->levels[0];
+    L.flushPending = false;
+    if (!L.dev.wrapped) return;
+    int differ = 0;
+    int* flag = reinterpret_cast<int*>(g->scratch);
+    ck(cudaMemsetAsync(flag, 0, sizeof(int), g->stream), "memset");
+    lbm::launchGhostsDiffer(L.dev, L.info.esotwistFlipper, g->stream, flag);
+    ck(cudaGetLastError(), "ghost check launch");
+    ck(cudaMemcpyAsync(&differ, flag, sizeof(int), cudaMemcpyDeviceToHost, g->stream), "copy");
+    ck(cudaStreamSynchronize(g->stream), "sync");
+    L.ghostsCurrent = differ == 0;
+}
+
 // Host bookkeeping of one step whose kernels ran inside a replayed graph.
 void advanceHostState(LevelState& L) {
+    if (L.dev.wrapped) L.flushPending = true;
     L.info.esotwistFlipper = !L.info.esotwistFlipper;
     L.info.iterationsFinished++;
     L.iterationsSinceTrackerReset++;
@@ -344,34 +390,39 @@ cudaGraphExec_t pairGraph(lbm_grids* g, int parity) {
     // capture changes no host state: save and restore the step bookkeeping
     std::vector<lbm::Info> saved;
     std::vector<int> savedReset;
+    const bool savedFlush = g->levels[0].flushPending, savedGhosts = g->levels[0].ghostsCurrent;
     for (LevelState& L : g->levels) {
         saved.push_back(L.info);
         savedReset.push_back(L.iterationsSinceTrackerReset);
     }
+    auto restore = [&] {
+        for (size_t l = 0; l < g->levels.size(); ++l) {
+            g->levels[l].info = saved[l];
+            g->levels[l].iterationsSinceTrackerReset = savedReset[l];
+        }
+        g->levels[0].flushPending = savedFlush;
+        g->levels[0].ghostsCurrent = savedGhosts;
+    };
     g->levels[0].info.esotwistFlipper = parity != 0;
     cudaStream_t user = g->stream;
     g->stream = g->captureStream;
     cudaGraph_t graph = nullptr;
     ck(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     try {
+        // steps of a running series: the ghosts of a wrapped level are current
+        g->levels[0].ghostsCurrent = true;
         updateAllGrids(g, 0);
         updateAllGrids(g, 0);
     } catch (...) {
         cudaStreamEndCapture(g->stream, &graph);
         if (graph) cudaGraphDestroy(graph);
         g->stream = user;
-        for (size_t l = 0; l < g->levels.size(); ++l) {
-            g->levels[l].info = saved[l];
-            g->levels[l].iterationsSinceTrackerReset = savedReset[l];
-        }
+        restore();
         throw;
     }
     const cudaError_t e = cudaStreamEndCapture(g->stream, &graph);
     g->stream = user;
-    for (size_t l = 0; l < g->levels.size(); ++l) {
-        g->levels[l].info = saved[l];
-        g->levels[l].iterationsSinceTrackerReset = savedReset[l];
-    }
+    restore();
     ck(e, "end capture");
     cudaGraphExec_t exec = nullptr;
     const cudaError_t ei = cudaGraphInstantiate(&exec, graph, 0);
@@ -381,12 +432,27 @@ cudaGraphExec_t pairGraph(lbm_grids* g, int parity) {
     return exec;
 }
 
-// Launch two steps of a grids object from its graph, on its stream.
+// Launch two steps of a grids object from its graph, on its stream (a wrapped
+// level's ghosts are current: needsGhostStep is false).
 void launchPair(lbm_grids* g) {
     const int parity = g->levels[0].info.esotwistFlipper ? 1 : 0;
     cudaGraphExec_t exec = pairGraph(g, parity);
     ck(cudaGraphLaunch(exec, g->stream), "graph launch");
     for (int k = 0; k < 2; ++k) advanceHostStep(g);
+}
+
+// `steps` coarse steps on the grid stream: step pairs from the graph where one
+// applies, and the ordinary state at the end.
+void runSteps(lbm_grids* g, int steps) {
+    int s = 0;
+    if (s < steps && needsGhostStep(g)) {
+        updateAllGrids(g, 0);
+        ++s;
+    }
+    if (graphable(g))
+        for (; s + 2 <= steps; s += 2) launchPair(g);
+    for (; s < steps; ++s) updateAllGrids(g, 0);
+    finishSteps(g);
 }
 
 struct DeviceWaitError : std::runtime_error {
@@ -430,6 +496,7 @@ int guarded(const char* where, const std::function<void()>& body) {
 
 struct lbm_batch {
     std::vector<lbm_grids*> members;
+    std::vector<lbm_grids*> wrapped;  // the members that step without ghosts, outside the packed tables
     int storage = LBM_STORE_F32;
     lbm::DevBatch dev{};
     lbm_batch_info info{};
@@ -454,7 +521,24 @@ struct lbm_batch {
 
 namespace {
 
-void batchStep(lbm_batch* b, bool flip, cudaStream_t s) { lbm::launchPackedStep(b->dev, b->storage, flip, s); }
+// One step of all members: the packed launches, and the ghost-free ones of the
+// dense periodic members.  A member whose ghosts are not current (first = true,
+// never inside a graph) steps on its own through the packed kernel as a batch
+// of one, so that what it computes does not depend on the other members.
+void batchStep(lbm_batch* b, bool flip, cudaStream_t s, bool first = false) {
+    if (b->dev.domainCount > 0) lbm::launchPackedStep(b->dev, b->storage, flip, s);
+    std::vector<const lbm::DevLevel*> levels;
+    for (lbm_grids* g : b->wrapped) {
+        LevelState& L = g->levels[0];
+        if (first && !L.ghostsCurrent) {
+            lbm::launchCollidePacked(L.dev, flip, s);
+            lbm::launchPeriodic(L.dev, !flip, s);
+        } else {
+            levels.push_back(&L.dev);
+        }
+    }
+    lbm::launchWrapped(levels.data(), static_cast<int>(levels.size()), flip, s);
+}
 
 // Graph of two packed steps starting at esotwist parity `parity`.
 cudaGraphExec_t batchPairGraph(lbm_batch* b, int parity) {
@@ -477,15 +561,27 @@ cudaGraphExec_t batchPairGraph(lbm_batch* b, int parity) {
 void batchAdvance(lbm_batch* b, int steps) {
     bool flip = b->members[0]->levels[0].info.esotwistFlipper;
     int s = 0;
+    for (lbm_grids* g : b->wrapped)
+        if (needsGhostStep(g) && steps > 0) s = 1;
+    if (s == 1) {
+        batchStep(b, flip, b->stream, true);
+        flip = !flip;
+    }
     if (graphable(b->members[0]))
         for (; s + 2 <= steps; s += 2) ck(cudaGraphLaunch(batchPairGraph(b, flip ? 1 : 0), b->stream), "graph launch");
     for (; s < steps; ++s) {
         batchStep(b, flip, b->stream);
         flip = !flip;
     }
+    for (lbm_grids* g : b->members) {
+        LevelState& L = g->levels[0];
+        const bool ghostStep = needsGhostStep(g);
+        for (int k = 0; k < steps; ++k) advanceHostState(L);
+        L.ghostsCurrent = true;
+        if (ghostStep && steps == 1) L.flushPending = false;  // its ghosts were copied
+        finishSteps(L, b->stream);
+    }
     ck(cudaGetLastError(), "batch launch");
-    for (lbm_grids* g : b->members)
-        for (int k = 0; k < steps; ++k) advanceHostState(g->levels[0]);
 }
 
 void batchCheckParity(const lbm_batch* b) {
@@ -780,6 +876,11 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
             d.perIndex = own(upload(H.perIndex, s));
             d.perSource = own(upload(H.perSource, s));
             d.perCount = static_cast<int>(H.perIndex.size());
+            // the ghost-free step stands beside the default collide-stream only:
+            // a variant chosen by LBM3_COLLIDE_KERNEL runs with ghost copies
+            d.wrapped = H.wrapped && lbm::collideVariant() == lbm::CollideVariant::Pair &&
+                        static_cast<unsigned long long>(n) * storageBytes(c->storage) < (1ULL << 32);  // 32-bit offsets
+            d.wrapSkip = own(upload(H.wrapSkip, s));
             {
                 std::vector<int4> seg(H.segCell.size());
                 for (size_t q = 0; q < seg.size(); ++q)
@@ -958,6 +1059,7 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
             ck(cudaMemcpyAsync(self, &L.dev, sizeof(lbm::DevLevel), cudaMemcpyHostToDevice, s), "descriptor copy");
         }
         ck(cudaStreamSynchronize(s), "build sync");
+        checkGhosts(g);
         if (fluidUpdates) *fluidUpdates = host.fluidUpdatesPerIteration;
         // the driver's hooks are evaluated during the build only
         g->c.open_bc_hook = nullptr;
@@ -988,10 +1090,7 @@ int lbm_set_stream(lbm_grids* g, void* stream) {
 int lbm_update_all_grids(lbm_grids* g, int steps) {
     if (!g || steps < 0) return fail(LBM_ERR_INVALID, "lbm_update_all_grids: bad argument");
     return guarded("lbm_update_all_grids", [&] {
-        int s = 0;
-        if (graphable(g))
-            for (; s + 2 <= steps; s += 2) launchPair(g);
-        for (; s < steps; ++s) updateAllGrids(g, 0);
+        runSteps(g, steps);
         ck(cudaGetLastError(), "step launch");
     });
 }
@@ -1006,7 +1105,7 @@ int lbm_update_batch(lbm_grids* const* grids, int count, int steps) {
         int s = 0;
         for (; s + 2 <= steps; s += 2)
             for (int q = 0; q < count; ++q) {
-                if (graphable(grids[q])) {
+                if (graphable(grids[q]) && !needsGhostStep(grids[q])) {
                     launchPair(grids[q]);
                 } else {
                     updateAllGrids(grids[q], 0);
@@ -1015,6 +1114,7 @@ int lbm_update_batch(lbm_grids* const* grids, int count, int steps) {
             }
         for (; s < steps; ++s)
             for (int q = 0; q < count; ++q) updateAllGrids(grids[q], 0);
+        for (int q = 0; q < count; ++q) finishSteps(grids[q]);
         ck(cudaGetLastError(), "step launch");
     });
 }
@@ -1045,14 +1145,23 @@ int lbm_batch_create(lbm_grids* const* grids, int count, lbm_batch** out) {
         std::vector<int> itemStart{0};
         std::vector<int> perStart{0};
         long long cells = 0;
-        for (int q = 0; q < count; ++q) {
-            const lbm::DevLevel& d = b->members[q]->levels[0].dev;
+        int ghosts = 0, items = 0;
+        for (lbm_grids* g : b->members) {
+            const lbm::DevLevel& d = g->levels[0].dev;
+            cells += d.cellCount;
+            ghosts += d.perCount;
+            items += lbm::pairItems(d);
+            if (d.wrapped) {
+                b->wrapped.push_back(g);
+                continue;
+            }
+            const int q = static_cast<int>(levels.size());
             levels.push_back(d);
             itemStart.push_back(itemStart.back() + lbm::pairItems(d));
             for (int i = 0; i < d.obChunkCount; ++i) open.push_back(make_int2(q, i));
             perStart.push_back(perStart.back() + d.perCount);
-            cells += d.cellCount;
         }
+        const int packed = static_cast<int>(levels.size());
         ck(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "stream");
         ck(cudaStreamCreateWithFlags(&b->captureStream, cudaStreamNonBlocking), "stream");
         ck(cudaEventCreateWithFlags(&b->sync, cudaEventDisableTiming), "event");
@@ -1061,11 +1170,11 @@ int lbm_batch_create(lbm_grids* const* grids, int count, lbm_batch** out) {
         auto own = [&](auto* p) { if (p) b->owned.push_back(p); return p; };
         lbm::DevBatch& D = b->dev;
         D.levels = own(upload(levels, b->stream));
-        D.domainCount = count;
+        D.domainCount = packed;
         D.itemStart = own(upload(itemStart, b->stream));
         D.collideCount = itemStart.back();
-        D.work = own(devAlloc<int>(count + 1));
-        ck(cudaMemsetAsync(D.work, 0, (count + 1) * sizeof(int), b->stream), "memset");
+        D.work = own(devAlloc<int>(packed + 1));
+        ck(cudaMemsetAsync(D.work, 0, (packed + 1) * sizeof(int), b->stream), "memset");
         D.openItems = open.empty() ? nullptr : own(upload(open, b->stream));
         D.openCount = static_cast<int>(open.size());
         D.periodicStart = own(upload(perStart, b->stream));
@@ -1073,10 +1182,11 @@ int lbm_batch_create(lbm_grids* const* grids, int count, lbm_batch** out) {
         ck(cudaStreamSynchronize(b->stream), "batch upload");
         b->info.domain_count = count;
         b->info.cells = cells;
-        b->info.collide_items = D.collideCount;
+        b->info.collide_items = items;
         b->info.open_chunks = D.openCount;
-        b->info.periodic_cells = D.periodicCount;
-        b->info.launches_per_step = (D.collideCount > 0) + (D.openCount > 0) + (D.periodicCount > 0);
+        b->info.periodic_cells = ghosts;
+        b->info.launches_per_step = (D.collideCount > 0) + (D.openCount > 0) + (D.periodicCount > 0) +
+                                    lbm::wrappedLaunches(static_cast<int>(b->wrapped.size()));
     });
     if (rc != LBM_OK) {
         delete b;
@@ -1142,10 +1252,7 @@ int lbm_time_steps_graph(lbm_grids* g, int steps, float* ms) {
             pairGraph(g, 1);
         }
         ck(cudaEventRecord(g->ev0, g->stream), "event");
-        int s = 0;
-        if (graphable(g))
-            for (; s + 2 <= steps; s += 2) launchPair(g);
-        for (; s < steps; ++s) updateAllGrids(g, 0);
+        runSteps(g, steps);
         ck(cudaEventRecord(g->ev1, g->stream), "event");
         ck(cudaEventSynchronize(g->ev1), "event sync");
         checkDeviceFlag(g);
@@ -1173,11 +1280,16 @@ int lbm_time_steps(lbm_grids* g, int steps, float* ms) {
             g->kernelEvents.push_back(e);
         }
         g->kernelEventsUsed = 0;
+        int endLaunches = 0;
         g->timingKernels = true;
         try {
             ck(cudaEventRecord(g->ev0, g->stream), "event");
+            const bool ghostStep = needsGhostStep(g);
             for (int s = 0; s < steps; ++s) updateAllGrids(g, 0);
+            finishSteps(g);
             ck(cudaEventRecord(g->ev1, g->stream), "event");
+            // a wrapped series ends with one exchange; its first step may copy ghosts
+            if (g->levels[0].dev.wrapped && steps > 0) endLaunches = ghostStep ? (steps > 1) + 1 : 1;
         } catch (...) {
             g->timingKernels = false;
             throw;
@@ -1194,7 +1306,7 @@ int lbm_time_steps(lbm_grids* g, int steps, float* ms) {
         }
         g->lastKernelMs = kernel;
         g->lastLaunches = g->kernelEventsUsed / 2;
-        g->lastStepKernels = 0;
+        g->lastStepKernels = endLaunches;
         for (size_t l = 0; l < g->levels.size(); ++l) {
             const LevelState& L = g->levels[l];
             g->lastStepKernels += (static_cast<long long>(steps) << L.info.gridID) * lbm::stepLaunchCount(L.dev);
@@ -1361,6 +1473,7 @@ int lbm_write_f(lbm_grids* g, int level, const float* host, size_t bytes) {
             lbm::launchScatterF(L.dev, g->stream, tmp);
             ck(cudaGetLastError(), "write launch");
             ck(cudaStreamSynchronize(g->stream), "sync");
+            checkGhosts(g);
         } catch (...) {
             cudaFree(tmp);
             throw;
@@ -1860,6 +1973,7 @@ int lbm_load_state(lbm_grids* g, const void* host, size_t bytes) {
             }
         }
         ck(cudaStreamSynchronize(g->stream), "sync");
+        checkGhosts(g);
     });
 }
 

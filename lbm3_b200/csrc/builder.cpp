@@ -987,6 +987,31 @@ void buildSegments(HostLevel& L) {
     }
 }
 
+bool ghostFreePeriodic(const HostLevel& L, std::vector<uint32_t>& skip) {
+    skip.clear();
+    const Info& in = L.info;
+    const long long nx = in.nx, ny = in.ny, nz = in.nz, n = in.cellCount;
+    const long long mx = nx - 2, my = ny - 2, mz = nz - 2;
+    if (in.gridID != 0 || mx < 2 || my < 2 || mz < 2 || n != nx * ny * nz) return false;
+    if (!L.openCells.empty() || !L.wallIndex.empty() || L.wallCellCount != 0) return false;
+    if (static_cast<long long>(L.perIndex.size()) != n - mx * my * mz) return false;
+    for (size_t q = 0; q < L.perIndex.size(); ++q) {
+        const int c = L.perIndex[q];
+        auto inside = [](long long v, long long m) { return v == 0 ? m : v == m + 1 ? 1 : v; };
+        const long long i = inside(c % nx, mx), j = inside(c / nx % ny, my), k = inside(c / (nx * ny), mz);
+        if (L.perSource[q] != i + nx * (j + ny * k)) return false;
+    }
+    if (L.rotorCells.empty()) return true;
+    skip.assign(static_cast<size_t>((mx * my * mz + 31) / 32), 0u);
+    for (int c : L.rotorCells) {
+        const long long i = c % nx, j = c / nx % ny, k = c / (nx * ny);
+        if (i < 2 || i > mx - 1 || j < 2 || j > my - 1 || k < 2 || k > mz - 1) return false;
+        const long long q = (i - 1) + mx * ((j - 1) + my * (k - 1));
+        skip[static_cast<size_t>(q >> 5)] |= 1u << (q & 31);
+    }
+    return true;
+}
+
 namespace {
 
 size_t denseIndex(const Info& in, int i, int j, int k) {
@@ -1385,6 +1410,8 @@ void buildDomain(const lbm_case& c, HostDomain& out) {
         if (l + 1 < NL) buildInterfaces(L, marks[l], out.levels[l + 1], marks[l + 1]);
         buildRotors(c, L);
         buildSegments(L);
+        L.wrapped = NL == 1 && ghostFreePeriodic(L, L.wrapSkip);
+        if (!L.wrapped) L.wrapSkip.clear();
     }
 
     out.fluidUpdatesPerIteration = 0;

@@ -82,6 +82,8 @@ struct HostLevel {
     std::vector<int> wallMap;
     // periodic ghost copies (PeriodicBCStruct)
     std::vector<int> perIndex, perSource;
+    bool wrapped = false;                // ghostFreePeriodic
+    std::vector<uint32_t> wrapSkip;      // its skip bits
     std::vector<OpenBCList> openBCs;
     std::vector<OpenBCCell> openCells;   // all IDs, in ID then cell order
     int wallCellCount = 0;
@@ -149,6 +151,15 @@ void buildRotors(const lbm_case& c, HostLevel& L);
 
 // Split the compressed rows into bulk segments (needs wallMap and rotorCell).
 void buildSegments(HostLevel& L);
+
+// Whether the ghost-free periodic step applies to a level: a dense block of
+// cells whose outermost layer are periodic ghosts on every face, one cell deep
+// and copied from the opposite interior cell, without walls or open cells,
+// and with rotor cells (skip: one bit per interior cell in k-j-i order, empty
+// without rotors) only where no neighbour is a ghost.  Then a ghost behaves
+// exactly as its source, and a population that would arrive from a ghost is
+// found in the slot of the cell's own periodic image instead.
+bool ghostFreePeriodic(const HostLevel& L, std::vector<uint32_t>& skip);
 
 // Build all tables of every level; throws std::runtime_error on an invalid
 // case (the reference's setup throws at the same points).

@@ -1773,6 +1773,212 @@ __global__ void __launch_bounds__(kBlock) periodicPacked(DevBatch b) {
     periodicCell<F, S>(b.levels[lo], idx - __ldg(b.periodicStart + lo));
 }
 
+// ---- ghost-free periodic step ------------------------------------------------
+// A dense periodic box needs no ghosts between steps.  Esotwist gives every
+// slot one owner per step, and a slot that a population reaches by leaving the
+// box belongs to a ghost: the periodic image, on that side, of the very cell
+// which the population has to enter.  So an interior cell at a boundary reads
+// the directions that come across it from its own image's slots (index + m
+// times the axis' index step for the low face, - m times it for the high one)
+// and writes all 27 values to its own slots as always; ghosts are neither
+// collided nor copied.  A ghost only ever repeats its source's collision, so
+// the interior evolves exactly as with ghost copies.  Once, after the last step
+// of a call, wrappedFlush moves the boundary values into their cells' own slots
+// and refreshes the ghosts, which restores the state every other kernel reads.
+//
+// Per step this drops the ghost-copy launch and the collision of the ghosts
+// (9.7% of a 66^3 grid).  The interior cells are numbered without the ghosts, so
+// every tile is full (128 cells: two rows of a 64^3 box, aligned with them)
+// and needs no descriptor; the lane's row and column come from two
+// multiply-high divisions.  One tile per CTA, no shared memory, no barrier and
+// no work counter: the hardware replaces each finished CTA at once.  Addresses
+// are a uniform 64-bit plane base plus a 32-bit byte offset per lane, shared by
+// the nine directions of one x sign (64-bit element addresses cost 5%; the
+// offset limits a plane to 4 GB, larger levels keep their ghosts).
+//
+// Step of a Taylor-Green box, collide-stream and ghost copy before, this kernel
+// now: 64^3 FP32 20.4 -> 12.5 us, 64^3 FP64 45 -> 20.2, 128^3 FP32 112 -> 84,
+// 160^3 FP16 189 -> 167, eight 64^3 FP16 137 -> 88.  FP32 and FP64 are bound by
+// memory (83% of the copy bandwidth at 128^3), FP16 by the FP32 arithmetic.
+// Ten or more CTAs of 64 threads per SM (96 registers and less) spill: 107 us
+// at 128^3.
+#if LBM3_PART(5)
+#ifndef LBM3_WRAP_MIN_BLOCKS
+#define LBM3_WRAP_MIN_BLOCKS 8
+#endif
+
+// Where the lane's cell reads: its index, and the image shifts by the sign of
+// each velocity component (0: none, 1: +1, 2: -1).
+struct WrapLane {
+    int cell;
+    int x[3], y[3], z[3];
+    bool edge;  // on a j or k face
+};
+
+template <class T> __device__ __forceinline__ WrapLane wrapLane(const WrapDomain<T>& g, int q) {
+    WrapLane w;
+    const int row = static_cast<int>(__umulhi(unsigned(q), g.divX) >> g.shiftX);
+    const int k = static_cast<int>(__umulhi(unsigned(row), g.divY) >> g.shiftY);
+    const int i = q - row * g.mx, j = row - k * g.my;
+    w.cell = (i + 1) + (j + 1) * g.nx + (k + 1) * g.nxy;
+    w.x[0] = w.y[0] = w.z[0] = 0;
+    w.x[1] = i == 0 ? g.mx : 0;
+    w.x[2] = i == g.mx - 1 ? -g.mx : 0;
+    w.y[1] = j == 0 ? g.my * g.nx : 0;
+    w.y[2] = j == g.my - 1 ? -g.my * g.nx : 0;
+    w.z[1] = k == 0 ? g.mz * g.nxy : 0;
+    w.z[2] = k == g.mz - 1 ? -g.mz * g.nxy : 0;
+    w.edge = j == 0 || j == g.my - 1 || k == 0 || k == g.mz - 1;
+    return w;
+}
+
+constexpr int signSlot(int c) { return c > 0 ? 1 : c < 0 ? 2 : 0; }
+
+// The 27 pre-collision values.  Only the x shift differs between the lanes of
+// an inner row, so a warp without a j or k face adds nothing per direction.
+template <bool F, class S, bool kEdge, class T, class Get>
+__device__ __forceinline__ void wrapLoad(const WrapDomain<T>& g, Get&& put, const WrapLane& w) {
+    const char* base = static_cast<const char*>(g.f);
+    constexpr unsigned B = sizeof(S);
+    const unsigned ix[3] = {unsigned(w.cell) * B, unsigned(w.cell + w.x[1]) * B, unsigned(w.cell + w.x[2]) * B};
+#pragma unroll
+    for (int d = 0; d < 27; ++d) {
+        const char* plane = base + (preSlot<F>(d) * g.stride + ((cx(d) < 0 ? 1 : 0) + (cy(d) < 0 ? g.nx : 0) +
+                                                             (cz(d) < 0 ? g.nxy : 0))) * (long long)(B);
+        unsigned at = ix[signSlot(cx(d))];
+        if (kEdge) at += unsigned(w.y[signSlot(cy(d))] + w.z[signSlot(cz(d))]) * B;
+        put(d, Store<S>::ld(reinterpret_cast<const S*>(plane + at)));
+    }
+}
+
+template <class S> constexpr int wrapThreads() { return sizeof(S) == 8 ? kTile : kHalf; }
+
+template <bool F, class S>
+__global__ void __launch_bounds__(wrapThreads<S>(), sizeof(S) == 8 ? 4 : LBM3_WRAP_MIN_BLOCKS)
+    stepWrapped(const __grid_constant__ WrapBatch<Real<S>> b) {
+    using T = Real<S>;
+    const int t = threadIdx.x;
+    int dom = 0;
+    while (dom + 1 < b.count && int(blockIdx.x) >= b.tileStart[dom + 1]) ++dom;
+    const WrapDomain<T>& g = b.dom[dom];
+    const int tile = blockIdx.x - b.tileStart[dom];
+    Dither D{0u};
+    if constexpr (sizeof(S) == 2) {
+        if (tile == 0 && t == 0) g.seed[F ? 0 : 1] = mix32(g.seed[F ? 1 : 0] + 0x6D2B79F5u);
+        D.seed = g.seed[F ? 1 : 0] ^ kSaltCollide;
+    }
+    S* base = static_cast<S*>(g.f);
+    const int q0 = tile * kTile + t;
+    if constexpr (sizeof(S) == 8) {
+        bool ok = q0 < g.cells;
+        if (ok && g.skip) ok = !(__ldg(g.skip + (q0 >> 5)) >> (q0 & 31) & 1u);
+        if (!ok) return;
+        const WrapLane w = wrapLane(g, q0);
+        T f[27];
+        wrapLoad<F, S, true>(g, [&](int d, T v) { f[d] = v; }, w);
+        collideCumulantT(f, g.coll, g.coll.lambda, g.gx, g.gy, g.gz);
+#pragma unroll
+        for (int d = 0; d < 27; ++d)
+            Store<S>::st(base + (postSlot<F>(d) * g.stride + ((cx(d) > 0 ? 1 : 0) + (cy(d) > 0 ? g.nx : 0) +
+                                                              (cz(d) > 0 ? g.nxy : 0))) + unsigned(w.cell),
+                         f[d]);
+    } else {
+        bool okA = q0 < g.cells, okB = q0 + kHalf < g.cells;
+        // lanes past the end read the last cell (their stores are masked)
+        const WrapLane a = wrapLane(g, min(q0, g.cells - 1)), c = wrapLane(g, min(q0 + kHalf, g.cells - 1));
+        if (g.skip) {
+            okA = okA && !(__ldg(g.skip + (q0 >> 5)) >> (q0 & 31) & 1u);
+            okB = okB && !(__ldg(g.skip + ((q0 + kHalf) >> 5)) >> (q0 & 31) & 1u);
+        }
+        Pair f[27];
+        if (__any_sync(0xffffffffu, a.edge || c.edge)) {
+            wrapLoad<F, S, true>(g, [&](int d, float v) { f[d].v.x = v; }, a);
+            wrapLoad<F, S, true>(g, [&](int d, float v) { f[d].v.y = v; }, c);
+        } else {
+            wrapLoad<F, S, false>(g, [&](int d, float v) { f[d].v.x = v; }, a);
+            wrapLoad<F, S, false>(g, [&](int d, float v) { f[d].v.y = v; }, c);
+        }
+        collideCumulantT(f, g.coll, g.coll.lambda, g.gx, g.gy, g.gz);
+        unsigned x = sizeof(S) == 2 ? mix32(D.cell(a.cell)) : 0u;
+        const unsigned toA = unsigned(a.cell) * unsigned(sizeof(S)), toB = unsigned(c.cell) * unsigned(sizeof(S));
+#pragma unroll
+        for (int d = 0; d < 27; ++d) {
+            char* plane = reinterpret_cast<char*>(base + (postSlot<F>(d) * g.stride +
+                                                          ((cx(d) > 0 ? 1 : 0) + (cy(d) > 0 ? g.nx : 0) +
+                                                           (cz(d) > 0 ? g.nxy : 0))));
+            S* pa = reinterpret_cast<S*>(plane + toA);
+            S* pb = reinterpret_cast<S*>(plane + toB);
+            if constexpr (sizeof(S) == 2) {
+                x = x * 1664525u + 1013904223u;  // as in storePair
+                Store<S>::st2R(pa, pb, f[d].v.x, f[d].v.y, x ^ (x >> 16), okA, okB);
+            } else {
+                if (okA) Store<S>::st(pa, f[d].v.x);
+                if (okB) Store<S>::st(pb, f[d].v.y);
+            }
+        }
+    }
+}
+
+// Whether every ghost holds exactly its source's values (*differ stays 0), the
+// state the wrapped step starts from: one thread per ghost, flipper F.
+template <bool F, class S>
+__global__ void __launch_bounds__(kBlock) ghostsDiffer(DevLevel g, int* differ) {
+    const int idx = blockIdx.x * kBlock + threadIdx.x;
+    if (idx >= g.perCount) return;
+    using Bits = std::conditional_t<sizeof(S) == 8, unsigned long long,
+                                    std::conditional_t<sizeof(S) == 4, unsigned, unsigned short>>;
+    const Bits* base = static_cast<const Bits*>(g.f);
+    int a[8], b[8];
+    decodeNbr(g, __ldg(g.perIndex + idx), a, nullptr);
+    decodeNbr(g, __ldg(g.perSource + idx), b, nullptr);
+    bool same = true;
+#pragma unroll
+    for (int d = 0; d < 27; ++d) {
+        const Bits* plane = base + preSlot<F>(d) * g.stride;
+        same = same && plane[a[preNbr(d)]] == plane[b[preNbr(d)]];
+    }
+    if (!same) *differ = 1;
+}
+
+// One thread per ghost: F is the flipper after the last wrapped step.  A value
+// whose crossed faces are exactly those of this ghost lies in this ghost and
+// moves to the source's own slot; the ghost's other values are copied from
+// where the source reads them.  Every slot is written by one thread, and no
+// slot that a thread writes is read by another.
+template <bool F, class S>
+__global__ void __launch_bounds__(kBlock) wrappedFlush(DevLevel g) {
+    const int idx = blockIdx.x * kBlock + threadIdx.x;
+    if (idx >= g.perCount) return;
+    const int ghost = __ldg(g.perIndex + idx), src = __ldg(g.perSource + idx);
+    const int nx = g.nx, nxy = g.nx * g.ny;
+    const int mx = g.nx - 2, my = g.ny - 2, mz = g.nz - 2;
+    const int i = src % nx, j = src / nx % g.ny, k = src / nxy;       // source (1 .. m)
+    const int gi = ghost % nx, gj = ghost / nx % g.ny, gk = ghost / nxy;
+    int nbGhost[8], nbSrc[8];
+    decodeNbr(g, ghost, nbGhost, nullptr);
+    decodeNbr(g, src, nbSrc, nullptr);
+    S* base = static_cast<S*>(g.f);
+    const long long stride = g.stride;
+    S v[27];
+#pragma unroll
+    for (int d = 0; d < 27; ++d) {
+        // faces that direction d comes across at the source
+        const int sx = cx(d) > 0 ? (i == 1 ? mx : 0) : cx(d) < 0 ? (i == mx ? -mx : 0) : 0;
+        const int sy = cy(d) > 0 ? (j == 1 ? my : 0) : cy(d) < 0 ? (j == my ? -my : 0) : 0;
+        const int sz = cz(d) > 0 ? (k == 1 ? mz : 0) : cz(d) < 0 ? (k == mz ? -mz : 0) : 0;
+        v[d] = base[preSlot<F>(d) * stride + nbSrc[preNbr(d)] + sx + sy * nx + sz * nxy];
+    }
+#pragma unroll
+    for (int d = 0; d < 27; ++d) {
+        const int sx = cx(d) > 0 ? (i == 1 ? mx : 0) : cx(d) < 0 ? (i == mx ? -mx : 0) : 0;
+        const int sy = cy(d) > 0 ? (j == 1 ? my : 0) : cy(d) < 0 ? (j == my ? -my : 0) : 0;
+        const int sz = cz(d) > 0 ? (k == 1 ? mz : 0) : cz(d) < 0 ? (k == mz ? -mz : 0) : 0;
+        const bool here = gi - i == sx && gj - j == sy && gk - k == sz;
+        base[preSlot<F>(d) * stride + (here ? nbSrc : nbGhost)[preNbr(d)]] = v[d];
+    }
+}
+#endif
+
 inline unsigned blocksFor(long long n) { return static_cast<unsigned>((n + kBlock - 1) / kBlock); }
 
 // Dispatch on the flipper; this translation unit holds the kernels of one
@@ -1955,10 +2161,68 @@ template <bool F, class S> struct RunScatter {
 
 #define LBM3_FN(name) LBM3_STEP_JOIN(name, LBM3_STEP_SUFFIX)
 
+#if LBM3_PART(5)
+// Multiplier and shift with n / d == umulhi(n, multiplier) >> shift for
+// 0 <= n < 2^31 and d >= 2: with 2^shift < d <= 2^(shift + 1), multiplier =
+// ceil(2^(32 + shift) / d) fits 32 bits, and the quotient before truncation is
+// above n / d by less than n / 2^(32 + shift) <= (1 / d) n / 2^31 < 1 / d.
+static void divider(int d, unsigned& multiplier, int& shift) {
+    shift = 0;
+    while ((2LL << shift) < d) ++shift;
+    multiplier = static_cast<unsigned>(((1ULL << (32 + shift)) + d - 1) / d);
+}
+
+void LBM3_FN(launchWrapped)(const DevLevel* const* levels, int count, bool flip, cudaStream_t s) {
+    using T = Real<StepStore>;
+    for (int first = 0; first < count; first += kWrapDomains) {
+        WrapBatch<T> b{};
+        b.count = std::min(count - first, kWrapDomains);
+        for (int q = 0; q < b.count; ++q) {
+            const DevLevel& g = *levels[first + q];
+            WrapDomain<T>& w = b.dom[q];
+            w.f = g.f;
+            w.seed = g.seed;
+            w.skip = g.wrapSkip;
+            w.stride = g.stride;
+            w.nx = g.nx;
+            w.nxy = g.nx * g.ny;
+            w.mx = g.nx - 2;
+            w.my = g.ny - 2;
+            w.mz = g.nz - 2;
+            divider(w.mx, w.divX, w.shiftX);
+            divider(w.my, w.divY, w.shiftY);
+            w.cells = w.mx * w.my * w.mz;
+            w.gx = g.gx;
+            w.gy = g.gy;
+            w.gz = g.gz;
+            w.coll = collConsts<T>(g);
+            b.tileStart[q + 1] = b.tileStart[q] + (w.cells + kTile - 1) / kTile;
+        }
+        const int tiles = b.tileStart[b.count];
+        flip ? stepWrapped<true, StepStore><<<tiles, wrapThreads<StepStore>(), 0, s>>>(b)
+             : stepWrapped<false, StepStore><<<tiles, wrapThreads<StepStore>(), 0, s>>>(b);
+    }
+}
+void LBM3_FN(launchWrappedFlush)(const DevLevel& g, bool flip, cudaStream_t s) {
+    flip ? wrappedFlush<true, StepStore><<<blocksFor(g.perCount), kBlock, 0, s>>>(g)
+         : wrappedFlush<false, StepStore><<<blocksFor(g.perCount), kBlock, 0, s>>>(g);
+}
+void LBM3_FN(launchGhostsDiffer)(const DevLevel& g, bool flip, cudaStream_t s, int* differ) {
+    flip ? ghostsDiffer<true, StepStore><<<blocksFor(g.perCount), kBlock, 0, s>>>(g, differ)
+         : ghostsDiffer<false, StepStore><<<blocksFor(g.perCount), kBlock, 0, s>>>(g, differ);
+}
+#endif
+
 #if LBM3_PART(1)
 void LBM3_FN(launchCollidePair)(const DevLevel& g, bool flip, cudaStream_t s) { dispatch<RunCollidePair>(g, flip, s); }
 #endif
 #if LBM3_PART(2)
+void LBM3_FN(launchRotorCells)(const DevLevel& g, bool flip, cudaStream_t s) {
+    if (g.rotorCellCount <= 0) return;
+    const int blocks = (g.rotorCellCount + kListBlock - 1) / kListBlock;
+    flip ? collideRotorList<true, StepStore><<<blocks, kListBlock, 0, s>>>(g)
+         : collideRotorList<false, StepStore><<<blocks, kListBlock, 0, s>>>(g);
+}
 void LBM3_FN(launchCollideOther)(const DevLevel& g, bool flip, cudaStream_t s, CollideVariant v) {
     dispatch<RunCollideOther>(g, flip, s, v);
 }
@@ -2006,6 +2270,7 @@ void LBM3_FN(launchPackedStep)(const DevBatch& b, bool flip, cudaStream_t s) {
 // storage-independent launchers live in the FP32 unit of part 4
 int stepLaunchCount(const DevLevel& g) {
     int n = 0;
+    if (g.wrapped) return 1 + (g.rotorCellCount > 0);
     const CollideVariant v = collideVariant();
     if (v == CollideVariant::Simple) n += g.cellCount > 0;
     else if (v == CollideVariant::Prefetch || v == CollideVariant::Pair || v == CollideVariant::Packed)

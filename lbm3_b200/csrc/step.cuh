@@ -46,6 +46,8 @@ struct DevLevel {
     const int* rowKP;
     const int* rowJKP;       // [rowCount]
     const int* wallMap;      // [cellCount]
+    int wrapped;             // the ghost-free periodic step applies (ghostFreePeriodic in builder.h)
+    const unsigned* wrapSkip;  // WrapDomain::skip
     const int* perIndex;     // [perCount]
     const int* perSource;
     int perCount;
@@ -124,6 +126,31 @@ struct DevBatch {
     int periodicCount;
 };
 
+// A dense periodic level as the ghost-free step sees it (stepWrapped in
+// step.cu): nx x ny x nz cells of which the outermost layer are periodic
+// ghosts; T is the arithmetic type.  Passed by value.
+template <class T> struct WrapDomain {
+    void* f;                  // populations [27][stride]
+    unsigned* seed;           // as DevLevel::seed
+    const unsigned* skip;     // one bit per interior cell that another kernel collides; null: none
+    long long stride;
+    int nx, nxy;              // index distance of the +j and +k neighbours
+    int mx, my, mz;           // interior cells per axis
+    unsigned divX, divY;      // multipliers and shifts of the divisions by mx and my
+    int shiftX, shiftY;
+    int cells;                // mx * my * mz
+    T gx, gy, gz;
+    CollisionConstsT<T> coll;
+};
+// Several such domains in one launch: tiles [tileStart[q], tileStart[q + 1])
+// of the grid belong to domain q.
+constexpr int kWrapDomains = 16;
+template <class T> struct WrapBatch {
+    int count;
+    int tileStart[kWrapDomains + 1];
+    WrapDomain<T> dom[kWrapDomains];
+};
+
 // One level's pass over the section image of a flow report
 // (getFlowReportGeneral, include/flowReportFunctions.h:96-262): the cells of
 // layer `lowerNormal` (blended with the next layer by `alpha` when
@@ -158,11 +185,11 @@ inline int pairItems(const DevLevel& g) {
 }
 
 // Collision constants in the arithmetic type T.
-template <class T> __device__ __forceinline__ const CollisionConstsT<T>& collConsts(const DevLevel& g);
-template <> __device__ __forceinline__ const CollisionConstsT<float>& collConsts<float>(const DevLevel& g) {
+template <class T> __host__ __device__ __forceinline__ const CollisionConstsT<T>& collConsts(const DevLevel& g);
+template <> __host__ __device__ __forceinline__ const CollisionConstsT<float>& collConsts<float>(const DevLevel& g) {
     return g.coll;
 }
-template <> __device__ __forceinline__ const CollisionConstsT<double>& collConsts<double>(const DevLevel& g) {
+template <> __host__ __device__ __forceinline__ const CollisionConstsT<double>& collConsts<double>(const DevLevel& g) {
     return g.coll64;
 }
 

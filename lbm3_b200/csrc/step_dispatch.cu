@@ -40,6 +40,23 @@ void launchCollideStream(const DevLevel& g, bool flip, cudaStream_t s) {
                         paired && (!pairFits(g) || g.storage == LBM_STORE_F64) ? CollideVariant::Prefetch : v)
     }
 }
+void launchCollidePacked(const DevLevel& g, bool flip, cudaStream_t s) {
+    LBM3_BY_STORAGE(launchCollidePair, g, flip, s)
+}
+void launchRotorCells(const DevLevel& g, bool flip, cudaStream_t s) {
+    LBM3_BY_STORAGE(launchRotorCells, g, flip, s)
+}
+void launchWrapped(const DevLevel* const* levels, int count, bool flip, cudaStream_t s) {
+    if (count <= 0) return;
+    const DevLevel& g = *levels[0];
+    LBM3_BY_STORAGE(launchWrapped, levels, count, flip, s)
+}
+void launchWrappedFlush(const DevLevel& g, bool flip, cudaStream_t s) {
+    LBM3_BY_STORAGE(launchWrappedFlush, g, flip, s)
+}
+void launchGhostsDiffer(const DevLevel& g, bool flip, cudaStream_t s, int* differ) {
+    LBM3_BY_STORAGE(launchGhostsDiffer, g, flip, s, differ)
+}
 void launchPeriodic(const DevLevel& g, bool flip, cudaStream_t s) { LBM3_BY_STORAGE(launchPeriodic, g, flip, s) }
 void launchInterface(const DevLevel& coarse, const DevLevel& fine, const DevInterface& I, bool flipCoarse,
                      bool flipFine, cudaStream_t s) {

@@ -1,0 +1,86 @@
+"""The ghost-free periodic step on the GPU against the oracle, which copies
+ghosts after every step: sizes below, at and past one 128-cell tile, boxes two
+cells thin, call lengths that mix single steps, step pairs and the first step
+of a state whose ghosts disagree, and every storage."""
+import math
+
+import numpy as np
+import pytest
+
+import lbm3_b200 as L
+from lbm3_b200 import _abi as A
+import oracle as O
+from helpers import FIELD_REL_L2, density_velocity_errors, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(dims, storage=A.LBM_STORE_F32):
+    """A smooth wave whose ghosts hold the same values as their sources up to rounding."""
+    c = L.periodic_box(*dims, nu_lattice=0.02, storage=storage)
+    c.gx = 1e-6
+
+    def initial(bc, i, j, k, info):
+        a, b, d = (2 * math.pi * v / n for v, n in zip((i, j, k), dims))
+        bc.dRho = 1e-3 * math.cos(a - b)
+        bc.ux, bc.uy, bc.uz = 0.03 * math.sin(b + d), 0.02 * math.cos(a), 0.025 * math.sin(a - d)
+    return L.set_hooks(c, initial_condition=initial)
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2), (6, 10, 4), (8, 4, 4), (34, 6, 2), (30, 14, 18)])
+def test_matches_oracle(dims):
+    c = _case(dims)
+    o = O.OracleGrid(c)
+    with L.build_grids(c) as g:
+        for steps in (1, 1, 2, 5):
+            g.update_all_grids(steps)
+            o.step(steps)
+            e_rho, e_u, d_rho = density_velocity_errors(g.macro(), o.macro())
+            assert e_rho < FIELD_REL_L2 and e_u < FIELD_REL_L2 and d_rho < 1e-6, (steps, e_rho, e_u, d_rho)
+        # the ghosts repeat their sources after every call
+        m = g.macro()
+        np.testing.assert_array_equal(m[:, g.array("periodic_index")], m[:, g.array("periodic_source")])
+        # a written state whose ghosts disagree steps with ghost copies first
+        f = o.populations()
+        f[:, 0] += np.float32(1e-4)
+        o.set_populations(f)
+        g.set_populations(f)
+        g.update_all_grids(3)
+        o.step(3)
+        e_rho, e_u, _ = density_velocity_errors(g.macro(), o.macro())
+        assert e_rho < FIELD_REL_L2 and e_u < FIELD_REL_L2, (e_rho, e_u)
+    o.close()
+
+
+@pytest.mark.parametrize("storage,tol", [(A.LBM_STORE_F64, 2e-6), (A.LBM_STORE_F16, 5e-3), (A.LBM_STORE_BF16, 4e-2)])
+def test_storages_agree(storage, tol):
+    """Against FP32 after 9 steps.  Rounding: FP32 keeps 2^-24 of a population
+    per step, FP16 2^-11, BF16 2^-8; 9 steps of independent errors on
+    velocities an order of magnitude below the populations' sum stay below
+    ten units of it."""
+    with L.build_grids(_case((30, 14, 18))) as a, L.build_grids(_case((30, 14, 18), storage)) as b:
+        a.update_all_grids(9)
+        b.update_all_grids(4)
+        b.update_all_grids(5)
+        assert rel_l2(b.macro()[1:4].reshape(-1), a.macro()[1:4].reshape(-1)) < tol
+
+
+def test_batch_of_periodic_members():
+    """More members than one launch holds, with a channel among them: each
+    ends where it ends as a batch of its own, from states whose ghosts agree
+    and states whose ghosts do not."""
+    def cases():
+        out = [_case((6 + 2 * (q % 4), 8, 4 + 2 * (q % 3)), A.LBM_STORE_F16) for q in range(17)]
+        return out + [L.periodic_box(10, 8, 6, ux=0.03, storage=A.LBM_STORE_F16),
+                      L.open_channel(16, 8, 8, storage=A.LBM_STORE_F16)]
+    grids = [L.build_grids(c) for c in cases()]
+    with L.PackedBatch(grids) as b:
+        for steps in (1, 2, 3):
+            b.update(steps)
+    for c, g in zip(cases(), grids):
+        with L.build_grids(c) as alone:
+            with L.PackedBatch([alone]) as b:
+                for steps in (1, 2, 3):
+                    b.update(steps)
+            np.testing.assert_array_equal(alone.populations(), g.populations())
+        g.close()
