@@ -1611,41 +1611,45 @@ __global__ void __launch_bounds__(kBlock) globalSums(DevLevel g, double* out) {
     }
 }
 
+// Macroscopic fields of cells [first, first + count), out[4][count].
 template <bool F, class S>
-__global__ void __launch_bounds__(kBlock) macroFields(DevLevel g, float* out) {
-    const int cell = blockIdx.x * kBlock + threadIdx.x;
-    if (cell >= g.cellCount) return;
+__global__ void __launch_bounds__(kBlock) macroFields(DevLevel g, int first, int count, float* out) {
+    const int at = blockIdx.x * kBlock + threadIdx.x;
+    if (at >= count) return;
+    const int cell = first + at;
     int nb[8];
     decodeNbr(g, cell, nb, nullptr);
     Real<S> f[27];
     readPre<F, S>(g, nb, f);
     Real<S> dRho, ux, uy, uz;
     macroFromF(f, dRho, ux, uy, uz);
-    const long long n = g.cellCount;
-    out[cell] = float(dRho);
-    out[n + cell] = float(ux);
-    out[2 * n + cell] = float(uy);
-    out[3 * n + cell] = float(uz);
+    const long long n = count;
+    out[at] = float(dRho);
+    out[n + at] = float(ux);
+    out[2 * n + at] = float(uy);
+    out[3 * n + at] = float(uz);
 }
 
 template <bool F, class S>
-__global__ void __launch_bounds__(kBlock) gatherF(DevLevel g, float* out) {
-    // raw slot copy: out[slot][cell] = f[slot][cell] as FP32 (planes are
-    // stride apart on the device, cellCount apart in the output)
-    const long long i = (long long)blockIdx.x * kBlock + threadIdx.x;
+__global__ void __launch_bounds__(kBlock) gatherF(DevLevel g, long long first, int count, float* out) {
+    // raw slot copy of values [first, first + count) of [27][cellCount] as FP32
+    // (planes are stride apart on the device, cellCount apart in the output)
+    const int at = blockIdx.x * kBlock + threadIdx.x;
+    if (at >= count) return;
+    const long long i = first + at;
     const long long n = g.cellCount;
-    if (i >= 27 * n) return;
     const long long slot = i / n, cell = i - slot * n;
-    out[i] = Store<S>::ld(static_cast<const S*>(g.f) + slot * g.stride + cell);
+    out[at] = Store<S>::ld(static_cast<const S*>(g.f) + slot * g.stride + cell);
 }
 
 template <class S>
-__global__ void __launch_bounds__(kBlock) scatterF(DevLevel g, const float* in) {
-    const long long i = (long long)blockIdx.x * kBlock + threadIdx.x;
+__global__ void __launch_bounds__(kBlock) scatterF(DevLevel g, long long first, int count, const float* in) {
+    const int at = blockIdx.x * kBlock + threadIdx.x;
+    if (at >= count) return;
+    const long long i = first + at;
     const long long n = g.cellCount;
-    if (i >= 27 * n) return;
     const long long slot = i / n, cell = i - slot * n;
-    Store<S>::st(static_cast<S*>(g.f) + slot * g.stride + cell, in[i]);
+    Store<S>::st(static_cast<S*>(g.f) + slot * g.stride + cell, in[at]);
 }
 
 #if LBM3_SHARED_UNIT
@@ -2142,18 +2146,18 @@ template <bool F, class S> struct RunGlobalSums {
     }
 };
 template <bool F, class S> struct RunMacro {
-    static void run(const DevLevel& g, cudaStream_t s, float* out) {
-        macroFields<F, S><<<blocksFor(g.cellCount), kBlock, 0, s>>>(g, out);
+    static void run(const DevLevel& g, cudaStream_t s, int first, int count, float* out) {
+        macroFields<F, S><<<blocksFor(count), kBlock, 0, s>>>(g, first, count, out);
     }
 };
 template <bool F, class S> struct RunGather {
-    static void run(const DevLevel& g, cudaStream_t s, float* out) {
-        gatherF<F, S><<<blocksFor(27LL * g.cellCount), kBlock, 0, s>>>(g, out);
+    static void run(const DevLevel& g, cudaStream_t s, long long first, int count, float* out) {
+        gatherF<F, S><<<blocksFor(count), kBlock, 0, s>>>(g, first, count, out);
     }
 };
 template <bool F, class S> struct RunScatter {
-    static void run(const DevLevel& g, cudaStream_t s, const float* in) {
-        scatterF<S><<<blocksFor(27LL * g.cellCount), kBlock, 0, s>>>(g, in);
+    static void run(const DevLevel& g, cudaStream_t s, long long first, int count, const float* in) {
+        scatterF<S><<<blocksFor(count), kBlock, 0, s>>>(g, first, count, in);
     }
 };
 
@@ -2245,12 +2249,18 @@ void LBM3_FN(launchInit)(const DevLevel& g, bool flip, cudaStream_t s, const flo
 void LBM3_FN(launchKineticEnergy)(const DevLevel& g, bool flip, cudaStream_t s, double* out) {
     dispatch<RunEnergy>(g, flip, s, out);
 }
-void LBM3_FN(launchMacro)(const DevLevel& g, bool flip, cudaStream_t s, float* out) { dispatch<RunMacro>(g, flip, s, out); }
+void LBM3_FN(launchMacro)(const DevLevel& g, bool flip, cudaStream_t s, int first, int count, float* out) {
+    dispatch<RunMacro>(g, flip, s, first, count, out);
+}
 void LBM3_FN(launchGlobalSums)(const DevLevel& g, bool flip, cudaStream_t s, double* out) {
     dispatch<RunGlobalSums>(g, flip, s, out);
 }
-void LBM3_FN(launchGatherF)(const DevLevel& g, cudaStream_t s, float* out) { dispatch<RunGather>(g, false, s, out); }
-void LBM3_FN(launchScatterF)(const DevLevel& g, cudaStream_t s, const float* in) { dispatch<RunScatter>(g, false, s, in); }
+void LBM3_FN(launchGatherF)(const DevLevel& g, cudaStream_t s, long long first, int count, float* out) {
+    dispatch<RunGather>(g, false, s, first, count, out);
+}
+void LBM3_FN(launchScatterF)(const DevLevel& g, cudaStream_t s, long long first, int count, const float* in) {
+    dispatch<RunScatter>(g, false, s, first, count, in);
+}
 void LBM3_FN(launchFlowImage)(const DevLevel& g, bool flip, cudaStream_t s, const FlowImagePass& a, float* img) {
     dispatch<RunFlowImage>(g, flip, s, a, img);
 }

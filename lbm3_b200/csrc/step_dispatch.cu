@@ -75,12 +75,18 @@ void launchInit(const DevLevel& g, bool flip, cudaStream_t s, const float4* macr
 void launchKineticEnergy(const DevLevel& g, bool flip, cudaStream_t s, double* out) {
     LBM3_BY_STORAGE(launchKineticEnergy, g, flip, s, out)
 }
-void launchMacro(const DevLevel& g, bool flip, cudaStream_t s, float* out) { LBM3_BY_STORAGE(launchMacro, g, flip, s, out) }
+void launchMacro(const DevLevel& g, bool flip, cudaStream_t s, int first, int count, float* out) {
+    LBM3_BY_STORAGE(launchMacro, g, flip, s, first, count, out)
+}
 void launchGlobalSums(const DevLevel& g, bool flip, cudaStream_t s, double* out) {
     LBM3_BY_STORAGE(launchGlobalSums, g, flip, s, out)
 }
-void launchGatherF(const DevLevel& g, cudaStream_t s, float* out) { LBM3_BY_STORAGE(launchGatherF, g, s, out) }
-void launchScatterF(const DevLevel& g, cudaStream_t s, const float* in) { LBM3_BY_STORAGE(launchScatterF, g, s, in) }
+void launchGatherF(const DevLevel& g, cudaStream_t s, long long first, int count, float* out) {
+    LBM3_BY_STORAGE(launchGatherF, g, s, first, count, out)
+}
+void launchScatterF(const DevLevel& g, cudaStream_t s, long long first, int count, const float* in) {
+    LBM3_BY_STORAGE(launchScatterF, g, s, first, count, in)
+}
 void launchFlowReport(const DevLevel& g, bool flip, cudaStream_t s, int plane, int layer, int h0, int h1, int v0,
                       int v1, double* out) {
     LBM3_BY_STORAGE(launchFlowReport, g, flip, s, plane, layer, h0, h1, v0, v1, out)

@@ -32,11 +32,13 @@ void launchOpenBoundary(const DevLevel& g, bool flip, cudaStream_t s);
 void launchOpenBoundaryInit(const DevLevel& g, bool flip, cudaStream_t s);
 void launchInit(const DevLevel& g, bool flip, cudaStream_t s, const float4* macro, float4 uniform);
 void launchKineticEnergy(const DevLevel& g, bool flip, cudaStream_t s, double* out);
-void launchMacro(const DevLevel& g, bool flip, cudaStream_t s, float* out);
+// fields of cells [first, first + count) as out[4][count]
+void launchMacro(const DevLevel& g, bool flip, cudaStream_t s, int first, int count, float* out);
 // FP64 sums over the fluid cells: {rho, dRho, rho ux, rho uy, rho uz, cells}
 void launchGlobalSums(const DevLevel& g, bool flip, cudaStream_t s, double* out);
-void launchGatherF(const DevLevel& g, cudaStream_t s, float* out);
-void launchScatterF(const DevLevel& g, cudaStream_t s, const float* in);
+// values [first, first + count) of the populations as FP32 [27][cellCount]
+void launchGatherF(const DevLevel& g, cudaStream_t s, long long first, int count, float* out);
+void launchScatterF(const DevLevel& g, cudaStream_t s, long long first, int count, const float* in);
 void launchWallForce(const DevLevel& g, int wallID, cudaStream_t s, double* out);
 void launchFlowReport(const DevLevel& g, bool flip, cudaStream_t s, int plane, int layer, int h0, int h1, int v0,
                       int v1, double* out);
@@ -79,10 +81,10 @@ void launchCollidePacked(const DevLevel& g, bool flip, cudaStream_t s);
     void launchOpenBoundaryInit##SUF(const DevLevel& g, bool flip, cudaStream_t s);                            \
     void launchInit##SUF(const DevLevel& g, bool flip, cudaStream_t s, const float4* macro, float4 uniform);   \
     void launchKineticEnergy##SUF(const DevLevel& g, bool flip, cudaStream_t s, double* out);                  \
-    void launchMacro##SUF(const DevLevel& g, bool flip, cudaStream_t s, float* out);                           \
+    void launchMacro##SUF(const DevLevel& g, bool flip, cudaStream_t s, int first, int count, float* out);     \
     void launchGlobalSums##SUF(const DevLevel& g, bool flip, cudaStream_t s, double* out);                     \
-    void launchGatherF##SUF(const DevLevel& g, cudaStream_t s, float* out);                                    \
-    void launchScatterF##SUF(const DevLevel& g, cudaStream_t s, const float* in);                              \
+    void launchGatherF##SUF(const DevLevel& g, cudaStream_t s, long long first, int count, float* out);        \
+    void launchScatterF##SUF(const DevLevel& g, cudaStream_t s, long long first, int count, const float* in);  \
     void launchFlowReport##SUF(const DevLevel& g, bool flip, cudaStream_t s, int plane, int layer, int h0,     \
                                int h1, int v0, int v1, double* out);                                           \
     void launchPackedStep##SUF(const DevBatch& b, bool flip, cudaStream_t s);                                   \
