@@ -1821,12 +1821,15 @@ __global__ void __launch_bounds__(kBlock) periodicPacked(DevBatch b) {
 // no work counter: the hardware replaces each finished CTA at once.  Addresses
 // are a uniform 64-bit plane base plus a 32-bit byte offset per lane, shared by
 // the nine directions of one x sign (64-bit element addresses cost 5%; the
-// offset limits a plane to 4 GB, larger levels keep their ghosts).
+// offset limits a plane to 4 GB, larger levels keep their ghosts).  The domain
+// of a batch is the grid's second dimension, so that the compiler knows its
+// parameters, and with them every plane base, to be uniform.
 //
 // Step of a Taylor-Green box, collide-stream and ghost copy before, this kernel
-// now: 64^3 FP32 20.4 -> 12.5 us, 64^3 FP64 45 -> 20.2, 128^3 FP32 112 -> 84,
-// 160^3 FP16 189 -> 167, eight 64^3 FP16 137 -> 88.  FP32 and FP64 are bound by
-// memory (83% of the copy bandwidth at 128^3), FP16 by the FP32 arithmetic.
+// now: 64^3 FP32 20.4 -> 10.8 us, 64^3 FP64 45 -> 18.5, 128^3 FP32 112 -> 79,
+// 160^3 FP16 189 -> 147, eight 64^3 FP16 137 -> 77.  FP32 and FP64 are bound by
+// memory (87% of the copy bandwidth at 128^3), FP16 by instruction issue (62% of
+// the slots, the FMA pipe 55% and the ALU pipe 47% active).
 // Ten or more CTAs of 64 threads per SM (96 registers and less) spill: 107 us
 // at 128^3.
 #if LBM3_PART(5)
@@ -1885,10 +1888,9 @@ __global__ void __launch_bounds__(wrapThreads<S>(), sizeof(S) == 8 ? 4 : LBM3_WR
     stepWrapped(const __grid_constant__ WrapBatch<Real<S>> b) {
     using T = Real<S>;
     const int t = threadIdx.x;
-    int dom = 0;
-    while (dom + 1 < b.count && int(blockIdx.x) >= b.tileStart[dom + 1]) ++dom;
-    const WrapDomain<T>& g = b.dom[dom];
-    const int tile = blockIdx.x - b.tileStart[dom];
+    const WrapDomain<T>& g = b.dom[blockIdx.y];
+    const int tile = blockIdx.x;
+    if (tile * kTile >= g.cells) return;  // a domain smaller than the launch's largest
     Dither D{0u};
     if constexpr (sizeof(S) == 2) {
         if (tile == 0 && t == 0) g.seed[F ? 0 : 1] = mix32(g.seed[F ? 1 : 0] + 0x6D2B79F5u);
@@ -1925,9 +1927,13 @@ __global__ void __launch_bounds__(wrapThreads<S>(), sizeof(S) == 8 ? 4 : LBM3_WR
             wrapLoad<F, S, false>(g, [&](int d, float v) { f[d].v.x = v; }, a);
             wrapLoad<F, S, false>(g, [&](int d, float v) { f[d].v.y = v; }, c);
         }
+        unsigned toA = unsigned(a.cell), toB = unsigned(c.cell);
         collideCumulantT(f, g.coll, g.coll.lambda, g.gx, g.gy, g.gz);
-        unsigned x = sizeof(S) == 2 ? mix32(D.cell(a.cell)) : 0u;
-        const unsigned toA = unsigned(a.cell) * unsigned(sizeof(S)), toB = unsigned(c.cell) * unsigned(sizeof(S));
+        forgetAddress(toA);
+        forgetAddress(toB);
+        unsigned x = sizeof(S) == 2 ? mix32(D.cell(int(toA))) : 0u;
+        toA *= unsigned(sizeof(S));
+        toB *= unsigned(sizeof(S));
 #pragma unroll
         for (int d = 0; d < 27; ++d) {
             char* plane = reinterpret_cast<char*>(base + (postSlot<F>(d) * g.stride +
@@ -2203,8 +2209,8 @@ void LBM3_FN(launchWrapped)(const DevLevel* const* levels, int count, bool flip,
     using T = Real<StepStore>;
     for (int first = 0; first < count; first += kWrapDomains) {
         WrapBatch<T> b{};
-        b.count = std::min(count - first, kWrapDomains);
-        for (int q = 0; q < b.count; ++q) {
+        int tiles = 0;
+        for (int q = 0; q < std::min(count - first, kWrapDomains); ++q) {
             const DevLevel& g = *levels[first + q];
             WrapDomain<T>& w = b.dom[q];
             w.f = g.f;
@@ -2223,11 +2229,11 @@ void LBM3_FN(launchWrapped)(const DevLevel* const* levels, int count, bool flip,
             w.gy = g.gy;
             w.gz = g.gz;
             w.coll = collConsts<T>(g);
-            b.tileStart[q + 1] = b.tileStart[q] + (w.cells + kTile - 1) / kTile;
+            tiles = std::max(tiles, (w.cells + kTile - 1) / kTile);
         }
-        const int tiles = b.tileStart[b.count];
-        flip ? stepWrapped<true, StepStore><<<tiles, wrapThreads<StepStore>(), 0, s>>>(b)
-             : stepWrapped<false, StepStore><<<tiles, wrapThreads<StepStore>(), 0, s>>>(b);
+        const dim3 grid(tiles, count - first < kWrapDomains ? count - first : kWrapDomains);
+        flip ? stepWrapped<true, StepStore><<<grid, wrapThreads<StepStore>(), 0, s>>>(b)
+             : stepWrapped<false, StepStore><<<grid, wrapThreads<StepStore>(), 0, s>>>(b);
     }
 }
 void LBM3_FN(launchWrappedFlush)(const DevLevel& g, bool flip, cudaStream_t s) {

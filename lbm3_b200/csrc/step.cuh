@@ -142,12 +142,9 @@ template <class T> struct WrapDomain {
     T gx, gy, gz;
     CollisionConstsT<T> coll;
 };
-// Several such domains in one launch: tiles [tileStart[q], tileStart[q + 1])
-// of the grid belong to domain q.
+// Several such domains in one launch, one per second grid index.
 constexpr int kWrapDomains = 16;
 template <class T> struct WrapBatch {
-    int count;
-    int tileStart[kWrapDomains + 1];
     WrapDomain<T> dom[kWrapDomains];
 };
 
