@@ -605,6 +605,43 @@ template <class T, int N> struct SpecialScratch {
     unsigned code[7][N];
 };
 
+// Weights of the interpolated bounceback by packed link code c (gamma = c / 254
+// within [0.01, 1]): (1 - gamma) / (1 + gamma) of the pre-collision value,
+// gamma / (1 + gamma) of the two collided ones, 1 / (1 + gamma) of the wall
+// term, evaluated in FP32 as the formula stands.  A table, because two
+// divisions per link are half of a wall-adjacent cell's arithmetic.
+struct alignas(16) LinkWeights {
+    float v[256][4];
+    constexpr LinkWeights() : v{} {
+        for (int c = 0; c < 256; ++c) {
+            const float q = static_cast<float>(c) / 254.f;
+            const float gamma = q < 0.01f ? 0.01f : q > 1.f ? 1.f : q;
+            const float invDen = 1.f / (1.f + gamma);
+            v[c][0] = (1.f - gamma) * invDen;
+            v[c][1] = gamma * invDen;
+            v[c][2] = invDen;
+            v[c][3] = 0.f;
+        }
+    }
+};
+__device__ const LinkWeights kLinkWeights = LinkWeights();
+
+template <class T>
+__device__ __forceinline__ void linkWeights(unsigned code, bool ibb, T& wPre, T& wPost, T& invDen) {
+    if constexpr (sizeof(T) == 4) {
+        const float4 w = __ldg(reinterpret_cast<const float4*>(kLinkWeights.v[code]));
+        wPre = ibb ? w.x : 0.5f * (1.f / 1.5f);
+        wPost = ibb ? w.y : 0.5f * (1.f / 1.5f);
+        invDen = ibb ? w.z : 1.f / 1.5f;
+    } else {
+        const T q = static_cast<T>(code) / T(254);
+        const T gamma = !ibb ? T(0.5) : q < T(0.01f) ? T(0.01f) : q > T(1) ? T(1) : q;
+        invDen = T(1) / (T(1) + gamma);
+        wPre = (T(1) - gamma) * invDen;
+        wPost = gamma * invDen;
+    }
+}
+
 // Cells outside the bulk segments, one thread per listed cell: wall-adjacent
 // fluid cells get the interpolated bounceback of Zhao & Yong (2017) with a
 // moving-wall term and momentum-exchange force
@@ -618,11 +655,15 @@ template <class T, int N> struct SpecialScratch {
 // link codes wait in shared memory (lane-private columns, so no barrier), and a link's
 // position in the packed codes is the population count of the lower links.
 // (Read per link from global memory instead, each linked direction was a
-// divergent branch with one or two dependent loads: a collide-stream launch of
-// a three-level sphere, 2,984 wall-adjacent cells on the finest of 59,000 to
-// 160,000 cells, took 28 us on average and takes 13.6; a 150x46x58 channel with
-// a body 39 and 20.)
-template <bool F, class S, bool kRotors, int N>
+// divergent branch with one or two dependent loads.)  The links are straight-line
+// code with their weights from a table, since one branch per direction leaves
+// each one's latency exposed.  A collide-stream launch of a three-level sphere,
+// 2,984 wall-adjacent cells on the finest of 59,000 to 160,000 cells, took 28 us
+// on average and takes 12.5; a 150x46x58 channel with a body 39 and 18.4.)
+//
+// kPaired: FP32 cells collide with the operations of a tile's lane (Single),
+// so that a domain comes out the same from the paired and the packed kernel.
+template <bool F, class S, bool kRotors, bool kPaired, int N>
 __device__ __forceinline__ void collideSpecialCell(const DevLevel& g, int cell, const int (&nb)[8],
                                                    const int* ijk, SpecialScratch<Real<S>, N>& sc, int t) {
     const int wm = __ldg(g.wallMap + cell);
@@ -654,7 +695,16 @@ __device__ __forceinline__ void collideSpecialCell(const DevLevel& g, int cell, 
         const int at[3] = {ijk[0], ijk[1], ijk[2]};
         cellRotorForcing<F, S>(g, at, wm, f, gx, gy, gz, lambda);
     }
-    collideCumulantT(f, collConsts<T>(g), lambda, gx, gy, gz);
+    if constexpr (kPaired) {
+        Single p[27];
+#pragma unroll
+        for (int d = 0; d < 27; ++d) p[d].v = f[d];
+        collideCumulantT(p, g.coll, lambda, gx, gy, gz);
+#pragma unroll
+        for (int d = 0; d < 27; ++d) f[d] = p[d].v;
+    } else {
+        collideCumulantT(f, collConsts<T>(g), lambda, gx, gy, gz);
+    }
     const Dither D = stepDither<F, S>(g, kSaltCollide);
     if (wm < 0) {
         writePost<F, S>(g, nb, f, D);
@@ -662,38 +712,42 @@ __device__ __forceinline__ void collideSpecialCell(const DevLevel& g, int cell, 
     }
     T dRho, ux, uy, uz;
     macroFromF(f, dRho, ux, uy, uz);
-    T fx = T(0), fy = T(0), fz = T(0);
+    T fx = T(0), fy = T(0), fz = T(0), fu = T(0);
     // a linked direction goes to the next pre-collision slot of its inverse
-    // (inside the wall cell), the others stream as usual
+    // (inside the wall cell), the others stream as usual; straight-line code, so
+    // that the directions overlap
     S* wbase = static_cast<S*>(g.f);
     const long long stride = g.stride;
     const unsigned cb = D.cell(cell);
+    const bool ibb = g.useIBB;
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
         T v = f[d];
         int slot = postSlot<F>(d);
-        if (d != 0 && ((wallData >> d) & 1u)) {
+        if (d != 0) {
+            const bool linked = (wallData >> d) & 1u;
             const int id = inv(d);
             const T eu = T(cx(id)) * uwx + T(cy(id)) * uwy + T(cz(id)) * uwz;
             const T wallTerm = T(6) * weightT<T>(id) * (T(1) + dRho) * eu;
-            T gamma = T(0.5);
-            if (g.useIBB) {
-                const int link = __popc(wallData & ((1u << d) - 2u));
-                const unsigned c8 = (sc.code[link >> 2][t] >> (8 * (link & 3))) & 255u;
-                const T q = static_cast<T>(c8) / T(254);
-                gamma = q < T(0.01f) ? T(0.01f) : q > T(1) ? T(1) : q;
-            }
-            const T fPre = sc.pre[d > 0 ? d - 1 : 0][t];
-            const T invDen = T(1) / (T(1) + gamma);
-            v = ((T(1) - gamma) * invDen) * fPre + (gamma * invDen) * f[id] + (gamma * invDen) * f[d] +
-                invDen * wallTerm;
-            fx += -f[d] * (T(cx(d)) - uwx) + v * (T(cx(id)) - uwx);
-            fy += -f[d] * (T(cy(d)) - uwy) + v * (T(cy(id)) - uwy);
-            fz += -f[d] * (T(cz(d)) - uwz) + v * (T(cz(id)) - uwz);
-            slot = F ? inv(d) : d;
+            const int link = __popc(wallData & ((1u << d) - 2u));  // links before this one, at most 25
+            const unsigned code = ibb && linked ? (sc.code[link >> 2][t] >> (8 * (link & 3))) & 255u : 0u;
+            T wPre, wPost, invDen;
+            linkWeights<T>(code, ibb, wPre, wPost, invDen);
+            const T r = wPre * sc.pre[d > 0 ? d - 1 : 0][t] + wPost * f[id] + wPost * f[d] + invDen * wallTerm;
+            // momentum exchange -f_d (c_d - u_w) + r (c_id - u_w), c_id = -c_d
+            const T sum = linked ? f[d] + r : T(0);
+            fx -= T(cx(d)) * sum;
+            fy -= T(cy(d)) * sum;
+            fz -= T(cz(d)) * sum;
+            fu += linked ? f[d] - r : T(0);
+            v = linked ? r : v;
+            slot = linked ? (F ? inv(d) : d) : slot;
         }
         stD(wbase + (long long)slot * stride + nb[postNbr(d)], v, D, cb, d);
     }
+    fx += fu * uwx;
+    fy += fu * uwy;
+    fz += fu * uwz;
     if (g.trackWallForce && !(wallData & 1u)) {
         g.wallForce[wm] = force[0] + double(fx);
         g.wallForce[nw + wm] = force[1] + double(fy);
@@ -702,21 +756,20 @@ __device__ __forceinline__ void collideSpecialCell(const DevLevel& g, int cell, 
 }
 
 // One entry {cell, jPlus, kPlus, jkPlus} of the special list.
-template <bool F, class S, int N>
+template <bool F, class S, bool kPaired, int N>
 __device__ __forceinline__ void collideListed(const DevLevel& g, int idx, SpecialScratch<Real<S>, N>& sc, int t) {
     if (idx >= g.specialCount) return;
     const int4 rows = __ldg(g.special + idx);
     int nb[8];
     rowNbr(g, rows, nb);
-    collideSpecialCell<F, S, false, N>(g, rows.x, nb, nullptr, sc, t);
+    collideSpecialCell<F, S, false, kPaired, N>(g, rows.x, nb, nullptr, sc, t);
 }
 
-// The same as a call, for the packed kernel: inlined there, the listed cells'
-// registers made its tile loop spill (104 against 101 us for eight 64^3
-// domains in FP16).
+// The same as a call: inlined, the listed cells' registers make the tile loop of
+// the paired kernels spill.
 template <bool F, class S, int N>
 __device__ __noinline__ void collideListedCall(const DevLevel& g, int idx, SpecialScratch<Real<S>, N>& sc, int t) {
-    collideListed<F, S, N>(g, idx, sc, t);
+    collideListed<F, S, true, N>(g, idx, sc, t);
 }
 
 constexpr int kListBlock = 64;
@@ -725,7 +778,7 @@ template <bool F, class S>
 __global__ void __launch_bounds__(kListBlock) collideList(DevLevel g) {
     __shared__ SpecialScratch<Real<S>, kListBlock> sc;
     advanceDither<F, S>(g);
-    collideListed<F, S>(g, blockIdx.x * kListBlock + threadIdx.x, sc, threadIdx.x);
+    collideListed<F, S, false>(g, blockIdx.x * kListBlock + threadIdx.x, sc, threadIdx.x);
 }
 
 // Cells a rotor can reach while it turns, one thread each: special-cell
@@ -739,7 +792,7 @@ __global__ void __launch_bounds__(kListBlock) collideRotorList(DevLevel g) {
     const int cell = __ldg(g.rotorCells + idx);
     int nb[8], ijk[3];
     decodeNbr(g, cell, nb, ijk);
-    collideSpecialCell<F, S, true, kListBlock>(g, cell, nb, ijk, sc, threadIdx.x);
+    collideSpecialCell<F, S, true, false, kListBlock>(g, cell, nb, ijk, sc, threadIdx.x);
 }
 
 // Work items of one launch: special chunks [0, S) first (kTile listed cells
@@ -766,7 +819,7 @@ __global__ void __launch_bounds__(kTile, LBM3_PREFETCH_MIN_BLOCKS) collidePrefet
     };
     int item = fetch();
     while (item < nSpecial) {
-        collideListed<F, S>(g, item * kTile + t, sc, t);
+        collideListed<F, S, false>(g, item * kTile + t, sc, t);
         item = fetch();
     }
     int4 dCur, dNext;
@@ -816,18 +869,13 @@ __global__ void __launch_bounds__(kTile, LBM3_PREFETCH_MIN_BLOCKS) collidePrefet
 // kernel is bounded by instruction issue, not by the FMA pipe), and the
 // second cell's 27 loads and 27 stores reuse the first cell's address with
 // an immediate offset.  Population offsets are 32-bit element indices
-// (27 x stride < 2^31; larger grids take collidePrefetch).  The CTA fetches
-// its next work item while the current tile's loads are in flight; with
-// LBM3_PAIR_PREFETCH the next tile's populations are also loaded into
-// registers during the current tile's collision.
+// (27 x stride < 2^31; larger grids take collidePrefetch).  The CTA
+// fetches its next work item while the current tile's loads are in flight.
 constexpr int kHalf = kTile / 2;
 static_assert(kHalf == kListedPerItem, "a work item of the paired kernels holds one listed cell per thread");
 
 #ifndef LBM3_PAIR_MIN_BLOCKS
 #define LBM3_PAIR_MIN_BLOCKS 8
-#endif
-#ifndef LBM3_PAIR_PREFETCH
-#define LBM3_PAIR_PREFETCH 0
 #endif
 
 // Element offset of direction q's pre- (Pre) or post-collision run for the
@@ -896,7 +944,7 @@ __device__ __forceinline__ void loadTilePair(const DevLevel& g, const int4& d, i
 }
 
 template <bool F, class S>
-__global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePair(DevLevel g) {
+__global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePair(const __grid_constant__ DevLevel g) {
     __shared__ int slot[2];
     __shared__ SpecialScratch<float, kHalf> sc;
     const int nSpecial = (g.specialCount + kHalf - 1) / kHalf;
@@ -904,44 +952,30 @@ __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePair(DevLe
     int parity = 0;
     advanceDither<F, S>(g);
     const Dither D = stepDither<F, S>(g, kSaltCollide);
-    // a CTA's first two items are its own (blockIdx and blockIdx + gridDim), so
-    // the first tile's loads wait for no atomic; the counter hands out the rest
-    const int G = gridDim.x;
+    // a CTA's first item is its own (blockIdx), so its loads wait for no atomic;
+    // the counter hands out the rest, one when the CTA is ready for it: a CTA
+    // with listed cells, which take the longest, must not hold a tile meanwhile
     auto fetch = [&]() {
-        if (t == 0) slot[parity] = 2 * G + atomicAdd(g.work, 1);
+        if (t == 0) slot[parity] = int(gridDim.x) + atomicAdd(g.work, 1);
         __syncthreads();
         const int v = slot[parity];
         parity ^= 1;
         return v;
     };
-    int item = blockIdx.x, next = item + G;
+    int item = blockIdx.x;
     while (item < nSpecial) {  // CTA-uniform
-        collideListed<F, S>(g, item * kHalf + t, sc, t);
-        item = next;
-        next = fetch();
+        collideListedCall<F, S>(g, item * kHalf + t, sc, t);
+        item = fetch();
     }
     int4 dCur;
     int lCur;
     loadDesc(g, item - nSpecial, dCur, lCur);
-#if LBM3_PAIR_PREFETCH
-    Pair fn[27];
-    loadTilePair<F, S>(g, dCur, t, lCur, fn);
-#endif
     while (lCur > 0) {  // CTA-uniform: lengths come from the shared descriptors
         Pair f[27];
-#if LBM3_PAIR_PREFETCH
-#pragma unroll
-        for (int q = 0; q < 27; ++q) f[q] = fn[q];
-#else
         loadTilePair<F, S>(g, dCur, t, lCur, f);
-#endif
         int4 dNext;
         int lNext;
-        loadDesc(g, next - nSpecial, dNext, lNext);
-        next = fetch();  // the atomic's latency overlaps the loads in flight
-#if LBM3_PAIR_PREFETCH
-        loadTilePair<F, S>(g, dNext, t, lNext, fn);
-#endif
+        loadDesc(g, fetch() - nSpecial, dNext, lNext);  // the atomic's latency overlaps the loads in flight
         collideCumulantT(f, g.coll, g.coll.lambda, g.gx, g.gy, g.gz);
         storePair<F, S>(g, dCur, t, lCur, f, D);
         dCur = dNext;
@@ -1749,8 +1783,8 @@ __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePacked(Dev
         while (item < count) {  // CTA-uniform: items come through shared memory
             int next;
             if (item < nSpecial) {  // CTA-uniform branch: both sides fetch once
-                next = fetch(dom);
                 collideListedCall<F, S>(sg, item * kHalf + t, sc, t);
+                next = fetch(dom);
             } else {
                 int4 d;
                 int l;
