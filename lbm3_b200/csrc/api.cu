@@ -160,6 +160,20 @@ struct lbm_plan {
 
 namespace {
 
+// A cell's record {cell, jPlus, kPlus, jkPlus} for the kernels, and the records
+// of the 2x2x2 block of cells up from it (bit 0 = i, bit 1 = j, bit 2 = k).
+int4 cellRecord(const lbm::HostLevel& H, int cell) {
+    const int kp = H.kPlus[cell];
+    return make_int4(cell, H.jPlus[cell], kp, H.jPlus[kp]);
+}
+void cellBlock(const lbm::HostLevel& H, int cell, std::vector<int4>& out) {
+    const int4 r = cellRecord(H, cell);
+    for (int row : {r.x, r.y, r.z, r.w}) {
+        out.push_back(cellRecord(H, row));
+        out.push_back(cellRecord(H, row + 1 < H.info.cellCount ? row + 1 : 0));
+    }
+}
+
 // Open-boundary chunks of the boundary kernel: cells grouped by outer normal
 // (table row), kOpenChunk per CTA.
 size_t openChunkCount(const lbm::HostLevel& H) {
@@ -210,7 +224,7 @@ unsigned long long levelBytes(const lbm::HostLevel& H, int storage) {
          bytes(sources, sizeof(int)) + bytes(4 * m, sizeof(float));  // cell, info, nbr, target, beta, source, refs
     b += bytes(openChunkCount(H), sizeof(int4)) + (m ? bytes(LBM_MBBC_NORMALS, mbbcTableBytes(storage)) : 0);
     b += m ? bytes(2, sizeof(int)) : 0;                             // device iteration counter
-    b += bytes(H.f2cIndex.size() + H.f2cChild.size() + H.c2fIndex.size() + H.c2fChild.size(), sizeof(int));
+    b += bytes(9 * H.f2cIndex.size() + 16 * H.c2fIndex.size(), sizeof(int4));  // interface records
     b += bytes(H.leftIndex.size() + H.leftParent.size() + H.leftNbr.size(), sizeof(int));  // interface lists
     if (H.info.gridID == 0)
         b += bytes(8, sizeof(double)) + bytes(1, sizeof(int)) + bytes(stagingSize(H.info.cellCount), sizeof(float));
@@ -939,10 +953,7 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
                 d.segLen = own(upload(H.segLen, s));
                 d.segCount = static_cast<int>(seg.size());
                 std::vector<int4> special(H.specialCells.size());
-                for (size_t q = 0; q < special.size(); ++q) {
-                    const int cell = H.specialCells[q], kp = H.kPlus[cell];
-                    special[q] = make_int4(cell, H.jPlus[cell], kp, H.jPlus[kp]);
-                }
+                for (size_t q = 0; q < special.size(); ++q) special[q] = cellRecord(H, H.specialCells[q]);
                 d.special = own(upload(special, s));
                 d.specialCount = static_cast<int>(H.specialCells.size());
                 d.rotorCells = own(upload(H.rotorCells, s));
@@ -1082,12 +1093,26 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
             L.c2fIndex = H.c2fIndex; L.c2fChild = H.c2fChild;
             L.leftIndex = H.leftIndex; L.leftParent = H.leftParent; L.leftNbr = H.leftNbr;
             lbm::DevInterface& I = L.itf;
-            I.f2cIndex = own(upload(H.f2cIndex, s));
-            I.f2cChild = own(upload(H.f2cChild, s));
+            const lbm::HostLevel& fine = host.levels[l + 1];
+            std::vector<int4> read, write;
+            for (size_t q = 0; q < H.f2cIndex.size(); ++q) {
+                cellBlock(fine, H.f2cChild[q], read);
+                write.push_back(cellRecord(H, H.f2cIndex[q]));
+            }
+            I.f2cRead = own(upload(read, s));
+            I.f2cWrite = own(upload(write, s));
             I.f2cCount = static_cast<int>(H.f2cIndex.size());
-            I.c2fIndex = own(upload(H.c2fIndex, s));
-            I.c2fChild = own(upload(H.c2fChild, s));
+            ck(cudaStreamSynchronize(s), "interface upload");
+            read.clear();
+            write.clear();
+            for (size_t q = 0; q < H.c2fIndex.size(); ++q) {
+                cellBlock(H, H.c2fIndex[q], read);
+                cellBlock(fine, H.c2fChild[q], write);
+            }
+            I.c2fRead = own(upload(read, s));
+            I.c2fWrite = own(upload(write, s));
             I.c2fCount = static_cast<int>(H.c2fIndex.size());
+            ck(cudaStreamSynchronize(s), "interface upload");
             I.leftIndex = own(upload(H.leftIndex, s));
             I.leftParent = own(upload(H.leftParent, s));
             I.leftNbr = own(upload(H.leftNbr, s));

@@ -162,12 +162,14 @@ struct FlowImagePass {
 
 // Interface lists between a coarse level and the next finer one
 // (InterfaceStruct, include/types.h:198-200) and the two levels' omega1.
+// Each item's cells as records {cell, jPlus, kPlus, jkPlus}, one per lane of its
+// group, so that a stencil cell's populations are one load away.
 struct DevInterface {
-    const int* f2cIndex;     // [f2cCount] coarse cell
-    const int* f2cChild;     // [f2cCount] its fine child (2i, 2j, 2k)
+    const int4* f2cRead;     // [f2cCount][8] the fine children (2i, 2j, 2k) and up
+    const int4* f2cWrite;    // [f2cCount] the coarse cell
     int f2cCount;
-    const int* c2fIndex;     // [c2fCount] -x-y-z coarse corner of a full stencil
-    const int* c2fChild;     // [c2fCount] fine cell (2i+1, 2j+1, 2k+1)
+    const int4* c2fRead;     // [c2fCount][8] the coarse cells of a full stencil, from its -x-y-z corner
+    const int4* c2fWrite;    // [c2fCount][8] the fine cells between them, from (2i+1, 2j+1, 2k+1)
     int c2fCount;
     const int* leftIndex;    // [leftCount] fine cell
     const int* leftParent;   // [leftCount] its coarse parent
