@@ -1009,6 +1009,10 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
                         chunks.push_back(make_int4(first + c0, std::min(lbm::kOpenChunk, count - c0), row,
                                                    static_cast<int>(tables[row].unknownMask)));
                 }
+                // the chunks on the x faces first: their gathers are the slowest
+                // (every value in a sector of its own), so they should not be the
+                // launch's last wave
+                std::stable_partition(chunks.begin(), chunks.end(), [&](const int4& c) { return tables[c.z].nx != 0; });
                 std::vector<int> cell(m), info(m), source;
                 std::vector<int4> nbr(m);
                 std::vector<float4> target(m);

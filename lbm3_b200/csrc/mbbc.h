@@ -12,8 +12,8 @@
 // formed in double and rounded once (equal to the generated code to
 // rounding).  The tables are stored transposed, column m (or d) holding the
 // weights of every unknown row, padded to kMbbcRowPad, so that a kernel
-// forms all rows at once: one 16-byte shared-memory load feeds four FMAs,
-// and the columns of unknown populations (zero weights) are skipped.  Populations are
+// forms all rows at once: one 16-byte shared-memory load feeds four FMAs
+// (the columns of unknown populations are zero).  Populations are
 // full (weight-compensated) f, as at the reference's call site
 // (include/updateGrid.h:223-240); restoreRho and restoreUxUyUz keep the
 // generated sums in ascending direction order.
@@ -134,20 +134,21 @@ LBM_HD void mbbcLoad4(const double* p, double (&o)[4]) {
 #endif
 }
 
-// applyMBBC for every unknown row at once: out[r] is the closed (full)
-// population T.unknownDir[r] for r < T.nu.  `unknown` is T.unknownMask (the
-// skipped columns) and `groups` = (T.nu + 3) / 4, both uniform over a CTA.
-template <class V>
-LBM_HD void mbbcClose(const MbbcDirT<V>& T, unsigned unknown, int groups, const V (&meq)[kMbbcMoments],
-                      const V (&f)[27], V (&out)[kMbbcRowPad]) {
+// applyMBBC for the unknown rows of 4 * kGroups: out[r] is the closed (full)
+// population T.unknownDir[r] for r < T.nu.  f is zero at the unknown
+// populations, whose columns are zero too, so the sweep is straight-line code:
+// its shared-memory loads overlap, where a branch per column and group of rows
+// left each load's latency exposed.
+template <int kGroups, class V>
+LBM_HD void mbbcCloseRows(const MbbcDirT<V>& T, const V (&meq)[kMbbcMoments], const V (&f)[27],
+                          V (&out)[kMbbcRowPad]) {
 #pragma unroll
-    for (int r = 0; r < kMbbcRowPad; ++r) out[r] = V(0);
+    for (int r = 0; r < 4 * kGroups; ++r) out[r] = V(0);
 #pragma unroll
     for (int m = 0; m < kMbbcMoments; ++m) {
         if (m == 10) continue;  // the moment is zero at equilibrium
 #pragma unroll
-        for (int q = 0; q < kMbbcRowPad / 4; ++q) {
-            if (q >= groups) break;
+        for (int q = 0; q < kGroups; ++q) {
             V w[4];
             mbbcLoad4(&T.ET[m][4 * q], w);
 #pragma unroll
@@ -156,16 +157,22 @@ LBM_HD void mbbcClose(const MbbcDirT<V>& T, unsigned unknown, int groups, const 
     }
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
-        if ((unknown >> d) & 1u) continue;
 #pragma unroll
-        for (int q = 0; q < kMbbcRowPad / 4; ++q) {
-            if (q >= groups) break;
+        for (int q = 0; q < kGroups; ++q) {
             V w[4];
             mbbcLoad4(&T.CT[d][4 * q], w);
 #pragma unroll
             for (int k = 0; k < 4; ++k) out[4 * q + k] = mfma(w[k], f[d], out[4 * q + k]);
         }
     }
+}
+
+// All unknown rows: nine on a face, up to nineteen on edges and corners
+// (uniform over a CTA).
+template <class V>
+LBM_HD void mbbcClose(const MbbcDirT<V>& T, const V (&meq)[kMbbcMoments], const V (&f)[27], V (&out)[kMbbcRowPad]) {
+    if (T.nu <= 12) mbbcCloseRows<3>(T, meq, f, out);
+    else mbbcCloseRows<5>(T, meq, f, out);
 }
 
 // restoreRho: density from the known populations and the velocity.

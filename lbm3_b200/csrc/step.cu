@@ -82,7 +82,6 @@ constexpr int kBlock = 256;
 // 27 pointers kept across the collision spill.
 __device__ __forceinline__ void forgetAddress(unsigned& offset) { asm volatile("" : "+r"(offset)); }
 
-
 // ---- rotors ---------------------------------------------------------------
 // Volume-fraction forcing towards rigid rotation (processRotor,
 // include/rotorFunctions.h:211-304, and its call in the cell update,
@@ -1316,8 +1315,9 @@ __device__ __forceinline__ V nonReflectiveUNormal(V uTarget, V dRhoZ, V dRhoRef)
 // their cells are disjoint and a cell touches only its own 27 slots, so the
 // reference's loop over IDs gives the same result in any order.
 #ifndef LBM3_OPEN_MIN_BLOCKS
-#define LBM3_OPEN_MIN_BLOCKS 8
+#define LBM3_OPEN_MIN_BLOCKS 6
 #endif
+template <class V> constexpr int openMinBlocks() { return sizeof(V) == 8 ? 4 : LBM3_OPEN_MIN_BLOCKS; }
 // The open-boundary launch's last CTA advances the device iteration count.
 __device__ __forceinline__ void openBoundaryDone(const DevLevel& g) {
     if (threadIdx.x == 0) {
@@ -1427,7 +1427,7 @@ __device__ __forceinline__ void openClose(const DevLevel& g, const MbbcDirT<Real
     {
         V meq[kMbbcMoments];
         mbbcMomentsEq(dRho + V(1), ux, uy, uz, meq);
-        mbbcClose(T, unknown, (T.nu + 3) >> 2, meq, c.f, closed);
+        mbbcClose(T, meq, c.f, closed);
     }
     const Dither D = stepDither<F, S>(g, kSaltOpen);
     const unsigned cb = D.cell(c.rows.x);
@@ -1494,7 +1494,7 @@ __device__ __forceinline__ void openBoundaryChunk(const DevLevel& g, int chunkIn
 
 // One chunk per CTA.
 template <bool F, class S>
-__global__ void __launch_bounds__(kOpenChunk, LBM3_OPEN_MIN_BLOCKS) openBoundary(DevLevel g) {
+__global__ void __launch_bounds__(kOpenChunk, openMinBlocks<Real<S>>()) openBoundary(DevLevel g) {
     __shared__ MbbcDirT<Real<S>> T;
     openBoundaryChunk<F, S>(g, blockIdx.x, T);
 }
@@ -1811,7 +1811,7 @@ __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePacked(Dev
 
 // One open-boundary chunk of one domain per CTA.
 template <bool F, class S>
-__global__ void __launch_bounds__(kOpenChunk, LBM3_OPEN_MIN_BLOCKS) openPacked(DevBatch b) {
+__global__ void __launch_bounds__(kOpenChunk, openMinBlocks<Real<S>>()) openPacked(DevBatch b) {
     __shared__ MbbcDirT<Real<S>> T;
     __shared__ DevLevel sg;
     const int2 it = __ldg(b.openItems + blockIdx.x);
