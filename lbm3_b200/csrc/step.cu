@@ -457,8 +457,13 @@ __device__ __forceinline__ void segNbr(const DevLevel& g, const int4& d, int t, 
     nb[7] = d.w + t + 1;
 }
 
+// Tile of a launch's q-th bulk item: up the domain at one esotwist parity, down
+// at the other, so that a step starts on the cells that the one before wrote
+// last, which the L2 cache (126 MB) still holds.  Past the end: out of range.
+template <bool F> __device__ __forceinline__ int sweep(int q, int count) { return F ? count - 1 - q : q; }
+
 __device__ __forceinline__ void loadDesc(const DevLevel& g, int tile, int4& d, int& l) {
-    if (tile < g.segCount) {
+    if (unsigned(tile) < unsigned(g.segCount)) {
         d = __ldg(g.seg + tile);
         l = __ldg(g.segLen + tile);
     } else {
@@ -1000,13 +1005,13 @@ __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePair(const
     }
     int4 dCur;
     int lCur;
-    loadDesc(g, item - nSpecial, dCur, lCur);
+    loadDesc(g, sweep<F>(item - nSpecial, g.segCount), dCur, lCur);
     while (lCur > 0) {  // CTA-uniform: lengths come from the shared descriptors
         Pair f[27];
         loadTilePair<F, S>(g, dCur, t, lCur, f);
         int4 dNext;
         int lNext;
-        loadDesc(g, fetch() - nSpecial, dNext, lNext);  // the atomic's latency overlaps the loads in flight
+        loadDesc(g, sweep<F>(fetch() - nSpecial, g.segCount), dNext, lNext);  // the atomic's latency overlaps the loads in flight
         collideCumulantT(f, g.coll, g.coll.lambda, g.gx, g.gy, g.gz);
         storePair<F, S>(g, dCur, t, lCur, f, D);
         dCur = dNext;
@@ -1822,7 +1827,7 @@ __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collidePacked(Dev
             } else {
                 int4 d;
                 int l;
-                loadDesc(sg, item - nSpecial, d, l);
+                loadDesc(sg, sweep<F>(item - nSpecial, sg.segCount), d, l);
                 Pair f[27];
                 loadTilePair<F, S>(sg, d, t, l, f);
                 next = fetch(dom);  // the atomic and the barrier overlap the tile's loads in flight
@@ -1958,8 +1963,8 @@ __global__ void __launch_bounds__(wrapThreads<S>(), sizeof(S) == 8 ? 4 : LBM3_WR
     gridWait();
     const int t = threadIdx.x;
     const WrapDomain<T>& g = b.dom[blockIdx.y];
-    const int tile = blockIdx.x;
-    if (tile * kTile >= g.cells) return;  // a domain smaller than the launch's largest
+    const int tile = sweep<F>(blockIdx.x, (g.cells + kTile - 1) / kTile);
+    if (tile < 0 || tile * kTile >= g.cells) return;  // a domain smaller than the launch's largest
     Dither D{0u};
     if constexpr (sizeof(S) == 2) {
         if (tile == 0 && t == 0) g.seed[F ? 0 : 1] = mix32(g.seed[F ? 1 : 0] + 0x6D2B79F5u);
