@@ -120,7 +120,8 @@ struct lbm_grids {
     std::vector<cudaEvent_t> forkEvents, joinEvents;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double* scratch = nullptr;
-    float* staging = nullptr;  // fields and populations pass through it on their way to and from the host
+    float* staging = nullptr;  // fields and populations pass through it on their way to and from the
+                               // host (behind the first level's populations, in their allocation)
     size_t stagingFloats = 0;
     int* errorFlag = nullptr;  // device word the kernels set when a bounded wait gives up
     float lastKernelMs = 0.f;
@@ -136,7 +137,6 @@ struct lbm_grids {
         for (auto& L : levels)
             for (void* p : L.owned) cudaFree(p);
         if (scratch) cudaFree(scratch);
-        if (staging) cudaFree(staging);
         if (errorFlag) cudaFree(errorFlag);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
@@ -893,7 +893,6 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
         g->scratch = devAlloc<double>(8);
         g->errorFlag = devAlloc<int>(1);
         g->stagingFloats = stagingSize(host.levels[0].info.cellCount);
-        g->staging = devAlloc<float>(g->stagingFloats);
         cudaStream_t s = g->stream;
         ck(cudaMemsetAsync(g->errorFlag, 0, sizeof(int), s), "memset");
         g->levels.resize(host.levels.size());
@@ -917,8 +916,13 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
             d.nx = H.info.nx; d.ny = H.info.ny; d.nz = H.info.nz;
             d.res = H.info.res; d.ox = H.info.ox; d.oy = H.info.oy; d.oz = H.info.oz;
             auto own = [&](auto* p) { if (p) L.owned.push_back(p); return p; };
-            // 256 bytes of tail so bulk copies rounded up to 16 bytes stay inside
-            d.f = own(devAlloc<unsigned char>(27ULL * d.stride * storageBytes(c->storage) + 256));
+            // 256 bytes of tail so bulk copies rounded up to 16 bytes stay inside; the
+            // planes are whole 128-byte lines, so the staging buffer behind is aligned
+            const size_t populationBytes = 27ULL * d.stride * storageBytes(c->storage) + 256;
+            unsigned char* planes = own(devAlloc<unsigned char>(
+                populationBytes + (l == 0 ? g->stagingFloats * sizeof(float) : 0)));
+            d.f = planes;
+            if (l == 0) g->staging = reinterpret_cast<float*>(planes + populationBytes);
             d.errorFlag = g->errorFlag;
             d.work = own(devAlloc<int>(2));
             ck(cudaMemsetAsync(d.work, 0, 2 * sizeof(int), s), "memset");
