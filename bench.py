@@ -444,9 +444,10 @@ def time_batch(cases, steps: int, warmup: int, torch) -> float:
 
 def time_packed(cases, steps: int, warmup: int) -> tuple:
     """MLUPS of independent single-level domains advanced as one packed batch
-    (one persistent collide-stream launch over the packed block table of all
-    of them, one open-boundary and one periodic launch per step, step pairs
-    replayed as a CUDA graph), device-timed on the batch stream; and the
+    (one launch per step for up to 16 periodic boxes; for other members one
+    persistent collide-stream launch over the packed block table, one
+    open-boundary and one periodic launch per step; step pairs replayed as a
+    CUDA graph), device-timed on the batch stream; and the
     batch's kernel launches per step."""
     import lbm3_b200 as L
     grids = [L.build_grids(c) for c in cases]
@@ -511,8 +512,8 @@ def storage_comparison(args, f32_value: float, torch) -> dict:
     out["batched_f16"] = {
         "value": round(batched, 2), "unit": "MLUPS",
         "workload": "8 Taylor-Green 64^3 domains (66^3 with ghosts), FP16-shifted, one packed batch: one "
-                    "persistent collide-stream launch over all domains' work items and one periodic-ghost "
-                    "launch per step, step pairs replayed as CUDA graphs",
+                    "launch of the ghost-free periodic step over all domains per step, step pairs replayed as "
+                    "CUDA graphs",
         "launches_per_step": launches,
         "plain_f32_single_domain": round(plain, 2),
         "ratio_vs_plain_f32_same_configuration": round(batched / plain, 4),

@@ -2,6 +2,7 @@
 //
 //   collideStream  K1: fused read -> cumulant collision -> esotwist write
 //                  (updateSingleGrid cell lambda, include/updateGrid.h:51-178)
+//   stepWrapped    K1 and K3 of a dense periodic box in one launch, without ghosts
 //   openBoundary   K2: moment-based open boundary on the streamed state (:181-355)
 //   periodicCopy   K3: ghost <- interior pre-collision copy (:358-382)
 //   interfaceExchange  K4-K6: fine-to-coarse, coarse-to-fine and leftover
