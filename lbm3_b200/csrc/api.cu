@@ -467,9 +467,33 @@ void launchPair(lbm_grids* g) {
     for (int k = 0; k < 2; ++k) advanceHostStep(g);
 }
 
+bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) (void)cudaGetLastError();
+    return status == cudaStreamCaptureStatusActive;
+}
+
+// A wrapped level whose stream a program is capturing: the program replays the
+// steps on states that are not known here, with ghosts that may differ from
+// their sources, so they are steps with ghost copies.
+bool capturedWrapped(const lbm_grids* g) { return g->levels[0].dev.wrapped && capturing(g->stream); }
+void captureSteps(lbm_grids* g, int steps) {
+    LevelState& L = g->levels[0];
+    const bool current = L.ghostsCurrent;  // the capture itself changes no state
+    for (int s = 0; s < steps; ++s) {
+        L.ghostsCurrent = false;
+        updateAllGrids(g, 0);
+    }
+    L.ghostsCurrent = current;
+}
+
 // `steps` coarse steps on the grid stream: step pairs from the graph where one
 // applies, and the ordinary state at the end.
 void runSteps(lbm_grids* g, int steps) {
+    if (capturedWrapped(g)) {
+        captureSteps(g, steps);
+        return;
+    }
     int s = 0;
     if (s < steps && needsGhostStep(g)) {
         updateAllGrids(g, 0);
@@ -583,16 +607,21 @@ struct lbm_batch {
 
 namespace {
 
+// Which dense periodic members of a batch copy ghosts in a step: none (steps of
+// a running series), those whose ghosts are not current (its first step), or
+// all (steps that a program captures, as in captureSteps).
+enum class GhostCopies { None, Stale, All };
+
 // One step of all members: the packed launches, and the ghost-free ones of the
-// dense periodic members.  A member whose ghosts are not current (first = true,
-// never inside a graph) steps on its own through the packed kernel as a batch
-// of one, so that what it computes does not depend on the other members.
-void batchStep(lbm_batch* b, bool flip, cudaStream_t s, bool first = false) {
+// dense periodic members.  A member that copies ghosts (never inside a graph of
+// the batch) steps on its own through the packed kernel as a batch of one, so
+// that what it computes does not depend on the other members.
+void batchStep(lbm_batch* b, bool flip, cudaStream_t s, GhostCopies copies = GhostCopies::None) {
     if (b->dev.domainCount > 0) lbm::launchPackedStep(b->dev, b->storage, flip, s);
     std::vector<const lbm::DevLevel*> levels;
     for (lbm_grids* g : b->wrapped) {
         LevelState& L = g->levels[0];
-        if (first && !L.ghostsCurrent) {
+        if (copies == GhostCopies::All || (copies == GhostCopies::Stale && !L.ghostsCurrent)) {
             lbm::launchCollidePacked(L.dev, flip, s);
             lbm::launchPeriodic(L.dev, !flip, s);
         } else {
@@ -623,10 +652,19 @@ cudaGraphExec_t batchPairGraph(lbm_batch* b, int parity) {
 void batchAdvance(lbm_batch* b, int steps) {
     bool flip = b->members[0]->levels[0].info.esotwistFlipper;
     int s = 0;
+    if (!b->wrapped.empty() && capturing(b->stream)) {
+        for (; s < steps; ++s, flip = !flip) batchStep(b, flip, b->stream, GhostCopies::All);
+        for (lbm_grids* g : b->members) {
+            for (int k = 0; k < steps; ++k) advanceHostState(g->levels[0]);
+            g->levels[0].flushPending = false;
+        }
+        ck(cudaGetLastError(), "batch launch");
+        return;
+    }
     for (lbm_grids* g : b->wrapped)
         if (needsGhostStep(g) && steps > 0) s = 1;
     if (s == 1) {
-        batchStep(b, flip, b->stream, true);
+        batchStep(b, flip, b->stream, GhostCopies::Stale);
         flip = !flip;
     }
     if (graphable(b->members[0]))
@@ -1188,7 +1226,9 @@ int lbm_update_batch(lbm_grids* const* grids, int count, int steps) {
         int s = 0;
         for (; s + 2 <= steps; s += 2)
             for (int q = 0; q < count; ++q) {
-                if (graphable(grids[q]) && !needsGhostStep(grids[q])) {
+                if (capturedWrapped(grids[q])) {
+                    captureSteps(grids[q], 2);
+                } else if (graphable(grids[q]) && !needsGhostStep(grids[q])) {
                     launchPair(grids[q]);
                 } else {
                     updateAllGrids(grids[q], 0);
@@ -1196,7 +1236,10 @@ int lbm_update_batch(lbm_grids* const* grids, int count, int steps) {
                 }
             }
         for (; s < steps; ++s)
-            for (int q = 0; q < count; ++q) updateAllGrids(grids[q], 0);
+            for (int q = 0; q < count; ++q) {
+                if (capturedWrapped(grids[q])) captureSteps(grids[q], 1);
+                else updateAllGrids(grids[q], 0);
+            }
         for (int q = 0; q < count; ++q) finishSteps(grids[q]);
         ck(cudaGetLastError(), "step launch");
     });

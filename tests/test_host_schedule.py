@@ -1,0 +1,124 @@
+"""Which kernels the C ABI runs on which states, checked without a GPU: the
+library's host objects on a device of host memory (drivers/host_device.cu),
+whose levels know when a kernel reads a state that it must not."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import pytest
+
+import lbm3_b200 as L
+from lbm3_b200 import _abi as A
+from lbm3_b200 import build as B
+
+ROOT = Path(__file__).resolve().parents[1]
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    B.build()
+    out = tmp_path_factory.mktemp("host") / "host_device.so"
+    objs = [str(B.OBJ_DIR / o) for o in ("api.o", "builder.o", "geometry.o")]
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-I/usr/local/cuda/include",
+                    "-Wl,-Bsymbolic", str(ROOT / "tests" / "drivers" / "host_device.cpp"), *objs, "-o", str(out)],
+                   check=True)
+    lib = C.CDLL(str(out))
+    for name, res, args in A.SIGNATURES:
+        fn = getattr(lib, name)
+        fn.restype, fn.argtypes = res, args
+    for name in ("cudaStreamBeginCapture", "cudaGraphLaunch", "cudaGraphInstantiate", "cudaStreamEndCapture"):
+        getattr(lib, name).restype = C.c_int
+    lib.host_device_pitch_limit.argtypes = [C.c_size_t]
+    return lib
+
+
+@pytest.fixture
+def device(library, monkeypatch):
+    """device(ghosts): an empty device whose new levels' ghosts repeat their sources, or do not."""
+    monkeypatch.setattr(A, "lib", lambda: library)
+
+    def reset(ghosts):
+        library.host_device_reset(int(ghosts))
+        return library
+    return reset
+
+
+def level(lib, order=0):
+    """{steps, ghosts repeat their sources, ghost exchange due, read in a wrong state}"""
+    out = (C.c_int * 4)()
+    assert lib.host_device_level(order, out) == 0
+    return dict(zip(("steps", "ghosts", "due", "wrong"), out))
+
+
+def done(steps):
+    """An ordinary state after `steps` steps, on which every kernel may run."""
+    return {"steps": steps, "ghosts": 1, "due": 0, "wrong": 0}
+
+
+class Captured:
+    """Work on `stream` inside the block is recorded; replay() runs it."""
+
+    def __init__(self, lib, stream):
+        self.lib, self.stream, self.exec = lib, C.c_void_p(stream), C.c_void_p()
+
+    def __enter__(self):
+        assert self.lib.cudaStreamBeginCapture(self.stream, 0) == 0
+        return self
+
+    def __exit__(self, *exc):
+        graph = C.c_void_p()
+        assert self.lib.cudaStreamEndCapture(self.stream, C.byref(graph)) == 0
+        assert self.lib.cudaGraphInstantiate(C.byref(self.exec), graph, C.c_ulonglong(0)) == 0
+
+    def replay(self):
+        assert self.lib.cudaGraphLaunch(self.exec, self.stream) == 0
+
+
+@pytest.mark.parametrize("ghosts", [False, True])
+@pytest.mark.parametrize("call", ["single", "pairs", "update_batch", "packed"])
+def test_captured_steps_replay_on_any_state(device, call, ghosts):
+    """A program's own graph of steps does not know the state that it is
+    replayed on: after new populations, their ghosts differ from their sources."""
+    lib = device(ghosts)
+    with L.build_grids(L.periodic_box(6, 4, 4)) as g:
+        g.set_stream(64)
+        batch = L.PackedBatch([g]) if call == "packed" else None
+        with Captured(lib, 64) as c:
+            if call == "single":
+                g.update_all_grids(1)
+                g.update_all_grids(1)
+            elif call == "pairs":
+                g.update_all_grids(2)
+            elif call == "update_batch":
+                L.update_batch([g], 2)
+            else:
+                batch.update(2)
+        assert level(lib)["steps"] == 0
+        for n in (1, 2):
+            g.set_populations(g.populations())
+            c.replay()
+            assert level(lib) == done(2 * n)
+        # and steps outside of it go on from there
+        g.update_all_grids(3)
+        assert level(lib) == done(7)
+        if batch:
+            batch.close()
+
+
+@pytest.mark.parametrize("ghosts", [False, True])
+@pytest.mark.parametrize("steps", [1, 2, 3, 4, 5])
+def test_states_between_calls(device, steps, ghosts):
+    """Every division of steps over the entry points leaves an ordinary state."""
+    lib = device(ghosts)
+    grids = [L.build_grids(L.periodic_box(6, 4, 4 + 2 * q)) for q in range(3)]
+    with L.PackedBatch(grids[1:]) as b:
+        for k in range(2):
+            grids[0].update_all_grids(steps)
+            b.update(steps)
+            L.update_batch(grids, steps)
+            for g in grids:
+                g.macro()
+                g.kinetic_energy(1.0, 1.0)
+            assert [level(lib, q) for q in range(3)] == [done(2 * (k + 1) * steps)] * 3
+    for g in grids:
+        g.close()
