@@ -650,6 +650,7 @@ cudaGraphExec_t batchPairGraph(lbm_batch* b, int parity) {
 
 // Advance `steps` packed steps on the batch stream (members already waited for).
 void batchAdvance(lbm_batch* b, int steps) {
+    if (steps == 0) return;  // the members' states, their ghosts among them, stay as they are
     bool flip = b->members[0]->levels[0].info.esotwistFlipper;
     int s = 0;
     if (!b->wrapped.empty() && capturing(b->stream)) {
@@ -662,7 +663,7 @@ void batchAdvance(lbm_batch* b, int steps) {
         return;
     }
     for (lbm_grids* g : b->wrapped)
-        if (needsGhostStep(g) && steps > 0) s = 1;
+        if (needsGhostStep(g)) s = 1;
     if (s == 1) {
         batchStep(b, flip, b->stream, GhostCopies::Stale);
         flip = !flip;

@@ -114,3 +114,22 @@ def test_captured_steps_replay_on_written_state(storage):
         ref.update_all_grids(4)
         np.testing.assert_allclose(g.macro(), ref.macro(), rtol=0, atol=2e-7)
         del graph
+
+
+def test_batch_timed_over_no_steps():
+    """A written state whose ghosts disagree, timed over no steps, then
+    advanced: as the oracle advances it."""
+    c = _case((8, 6, 4))
+    o = O.OracleGrid(c)
+    f = o.populations()
+    f *= 1 + 1e-2 * np.random.default_rng(3).standard_normal(f.shape).astype(np.float32)
+    o.set_populations(f)
+    with L.build_grids(c) as g:
+        g.set_populations(f)
+        with L.PackedBatch([g]) as b:
+            b.time_steps(0)
+            b.update(3)
+        o.step(3)
+        e_rho, e_u, _ = density_velocity_errors(g.macro(), o.macro())
+        assert e_rho < FIELD_REL_L2 and e_u < FIELD_REL_L2, (e_rho, e_u)
+    o.close()

@@ -122,3 +122,16 @@ def test_states_between_calls(device, steps, ghosts):
             assert [level(lib, q) for q in range(3)] == [done(2 * (k + 1) * steps)] * 3
     for g in grids:
         g.close()
+
+
+@pytest.mark.parametrize("call", ["update", "time_steps"])
+def test_no_steps_change_nothing(device, call):
+    """A batch advanced by no steps: ghosts that differ from their sources
+    still differ, and the next step copies them."""
+    lib = device(False)
+    with L.build_grids(L.periodic_box(6, 4, 4)) as g, L.build_grids(L.open_channel(8, 6, 6)) as other:
+        with L.PackedBatch([g, other]) as b:
+            getattr(b, call)(0)
+            assert (level(lib)["steps"], level(lib)["ghosts"]) == (0, 0)
+            b.update(2)
+        assert level(lib) == done(2)
