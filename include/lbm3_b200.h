@@ -227,7 +227,7 @@ typedef struct lbm_case {
     float tgv_length;           /* X = x / tgv_length (x in mm)                */
 
     /* getLocalBC (uniform over the domain) */
-    float collision_limiter;    /* BCStruct.collisionLimiter; <= 0 selects AllOne */
+    float collision_limiter;    /* BCStruct.collisionLimiter; <= 0 selects AllOne, infinite no limit */
     float nu_multiplier;        /* BCStruct.nuMultiplier                       */
     float gx, gy, gz;           /* BCStruct.gx/gy/gz body force, lattice units */
     int   use_ibb;              /* BCStruct.useIBB: 1 interpolated, 0 gamma=1/2 */

@@ -42,7 +42,7 @@ template <class T> struct CollisionConstsT {
     T omega1;      // 1 / (3 nu nuMultiplier + 1/2)
     T omega3, omega4, omega5, A, B;  // K17 parameters (:241-262)
     T tauTerm;     // 1/omega1 - 1/2
-    T lambda;      // collision limiter (K17 when > 0 and nuMultiplier <= 1)
+    T lambda;      // collision limiter, at most 1e30 (K17 when > 0 and nuMultiplier <= 1)
     int useK17;
     // products of the above that every cell needs
     T mHalfW1;     // -omega1 * 0.5
@@ -81,7 +81,10 @@ template <class T> inline CollisionConstsT<T> makeCollisionConstsT(T nu, T nuMul
            T(2) * omega2 * omega2 * (T(2) + T(9) * omega1 * (omega1 - T(2)))) /
           (T(3) * (omega1 - omega2) * (omega2 * (T(2) + T(3) * omega1) - T(8) * omega1));
     k.tauTerm = T(1) / omega1 - T(0.5);
-    k.lambda = limiter;
+    // an infinite limiter (none) makes (1 - omega) lambda v / (lambda + |v|) a
+    // quotient of infinities, and the reciprocal of 2^126 or more flushes to
+    // zero; 1e30 is above any |v| by more than FP64 resolves
+    k.lambda = limiter < T(1e30) ? limiter : T(1e30);
     k.useK17 = (limiter > T(0)) && (nuMultiplier <= T(1));
     k.mHalfW1 = -omega1 * T(0.5);
     k.w1x15 = T(1.5) * omega1;
