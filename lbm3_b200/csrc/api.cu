@@ -10,6 +10,7 @@
 #include <cstring>
 #include <exception>
 #include <functional>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -123,7 +124,9 @@ struct lbm_grids {
     float* staging = nullptr;  // fields and populations pass through it on their way to and from the
                                // host (behind the first level's populations, in their allocation)
     size_t stagingFloats = 0;
-    int* errorFlag = nullptr;  // device word the kernels set when a bounded wait gives up
+    std::mutex stagingLock;    // one transfer at a time, also from several host threads
+    int* errorFlag = nullptr;  // device word the kernels set when a bounded wait gives up; the next one
+                               // is checkGhosts' own
     float lastKernelMs = 0.f;
     int lastLaunches = 0;
     long long lastStepKernels = 0;  // every kernel launch of the last lbm_time_steps
@@ -227,7 +230,7 @@ unsigned long long levelBytes(const lbm::HostLevel& H, int storage) {
     b += bytes(9 * H.f2cIndex.size() + 16 * H.c2fIndex.size(), sizeof(int4));  // interface records
     b += bytes(H.leftIndex.size() + H.leftParent.size() + H.leftNbr.size(), sizeof(int));  // interface lists
     if (H.info.gridID == 0)
-        b += bytes(8, sizeof(double)) + bytes(1, sizeof(int)) + bytes(stagingSize(H.info.cellCount), sizeof(float));
+        b += bytes(8, sizeof(double)) + bytes(2, sizeof(int)) + bytes(stagingSize(H.info.cellCount), sizeof(float));
     return b;
 }
 
@@ -332,7 +335,7 @@ void checkGhosts(lbm_grids* g) {
     L.flushPending = false;
     if (!L.dev.wrapped) return;
     int differ = 0;
-    int* flag = reinterpret_cast<int*>(g->scratch);
+    int* flag = g->errorFlag + 1;
     ck(cudaMemsetAsync(flag, 0, sizeof(int), g->stream), "memset");
     lbm::launchGhostsDiffer(L.dev, L.info.esotwistFlipper, g->stream, flag);
     ck(cudaGetLastError(), "ghost check launch");
@@ -505,9 +508,28 @@ void runSteps(lbm_grids* g, int steps) {
     finishSteps(g);
 }
 
+// The staging buffer, held by one transfer; the grid stream is idle when it is
+// given back, also when the transfer failed.
+class StagingUse {
+    std::lock_guard<std::mutex> hold_;
+    cudaStream_t stream_;
+    bool busy_ = true;
+
+public:
+    explicit StagingUse(lbm_grids* g) : hold_(g->stagingLock), stream_(g->stream) {}
+    void finish() {
+        busy_ = false;
+        ck(cudaStreamSynchronize(stream_), "sync");
+    }
+    ~StagingUse() {
+        if (busy_) cudaStreamSynchronize(stream_);
+    }
+};
+
 // A level's macroscopic fields (float [4][cellCount]) to the host, piece by
 // piece through the staging buffer, in stream order; the stream is idle afterwards.
 void readMacro(lbm_grids* g, LevelState& L, float* host) {
+    StagingUse staging(g);
     const int n = L.dev.cellCount, piece = static_cast<int>(g->stagingFloats / 4);
     for (int first = 0; first < n; first += std::min(piece, n - first)) {
         const int count = std::min(piece, n - first);
@@ -519,11 +541,12 @@ void readMacro(lbm_grids* g, LevelState& L, float* host) {
             ck(cudaMemcpy2DAsync(host + first, size_t(n) * sizeof(float), g->staging, row, row, 4,
                                  cudaMemcpyDeviceToHost, g->stream), "copy");
     }
-    ck(cudaStreamSynchronize(g->stream), "sync");
+    staging.finish();
 }
 
 // A level's populations as FP32 [27][cellCount] to or from the host, likewise.
 template <bool kRead, class T> void copyPopulations(lbm_grids* g, LevelState& L, T* host) {
+    StagingUse staging(g);
     const long long total = 27LL * L.dev.cellCount, piece = static_cast<long long>(g->stagingFloats);
     for (long long first = 0; first < total; first += piece) {
         const int count = static_cast<int>(std::min(piece, total - first));
@@ -538,7 +561,7 @@ template <bool kRead, class T> void copyPopulations(lbm_grids* g, LevelState& L,
             ck(cudaGetLastError(), "write launch");
         }
     }
-    ck(cudaStreamSynchronize(g->stream), "sync");
+    staging.finish();
 }
 
 struct DeviceWaitError : std::runtime_error {
@@ -930,7 +953,7 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
         ck(cudaEventCreate(&g->ev0), "cudaEventCreate");
         ck(cudaEventCreate(&g->ev1), "cudaEventCreate");
         g->scratch = devAlloc<double>(8);
-        g->errorFlag = devAlloc<int>(1);
+        g->errorFlag = devAlloc<int>(2);
         g->stagingFloats = stagingSize(host.levels[0].info.cellCount);
         cudaStream_t s = g->stream;
         ck(cudaMemsetAsync(g->errorFlag, 0, sizeof(int), s), "memset");

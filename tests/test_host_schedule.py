@@ -3,8 +3,10 @@ library's host objects on a device of host memory (drivers/host_device.cu),
 whose levels know when a kernel reads a state that it must not."""
 import ctypes as C
 import subprocess
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 import lbm3_b200 as L
@@ -135,3 +137,17 @@ def test_no_steps_change_nothing(device, call):
             assert (level(lib)["steps"], level(lib)["ghosts"]) == (0, 0)
             b.update(2)
         assert level(lib) == done(2)
+
+
+def test_two_threads_read_one_object(device):
+    """Fields and populations of the levels of one object, read by two host
+    threads at once, each come out as from one thread."""
+    lib = device(True)
+    with L.build_grids(L.taylor_green_refined(16).case) as g:
+        reads = [lambda: g.macro(0), lambda: g.populations(1), lambda: g.macro(1)]
+        alone = [r() for r in reads]
+        lib.host_device_copy_delay(2000)  # between a read's kernel and its copy
+        with ThreadPoolExecutor(3) as pool:
+            for _ in range(3):
+                for a, b in zip(alone, pool.map(lambda r: r(), reads)):
+                    np.testing.assert_array_equal(a, b)
