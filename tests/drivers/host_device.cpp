@@ -99,6 +99,12 @@ void __cudaUnregisterFatBinary(void**) {}
 
 // ---- the runtime -------------------------------------------------------------
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
+    if (a != cudaDevAttrMaxPitch) return cudaErrorInvalidValue;
+    *v = static_cast<int>(pitchLimit);
+    return cudaSuccess;
+}
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "host device"; }
 cudaError_t cudaMalloc(void** p, size_t n) { *p = std::calloc(n ? n : 1, 1); return *p ? cudaSuccess : cudaErrorMemoryAllocation; }

@@ -151,3 +151,14 @@ def test_two_threads_read_one_object(device):
             for _ in range(3):
                 for a, b in zip(alone, pool.map(lambda r: r(), reads)):
                     np.testing.assert_array_equal(a, b)
+
+
+def test_fields_wider_than_a_pitched_copy(device):
+    """Fields of several staging pieces whose row is longer than the pitch that
+    a 2D copy may have (2^31 - 1 bytes; here 1 MiB, for a level that fits a test)."""
+    device(True).host_device_pitch_limit(1 << 20)
+    with L.build_grids(L.periodic_box(64, 64, 64)) as g:
+        m = g.macro()
+        assert m[0].nbytes > 1 << 20
+        cells = np.arange(m.shape[1], dtype=np.float32) * 16
+        np.testing.assert_array_equal(m, cells + 4 * np.arange(4, dtype=np.float32)[:, None])
