@@ -492,20 +492,25 @@ void captureSteps(lbm_grids* g, int steps) {
 }
 
 // `steps` coarse steps on the grid stream: step pairs from the graph where one
-// applies, and the ordinary state at the end.
+// applies, and the ordinary state at the end, also of a series that fails.
 void runSteps(lbm_grids* g, int steps) {
     if (capturedWrapped(g)) {
         captureSteps(g, steps);
         return;
     }
-    int s = 0;
-    if (s < steps && needsGhostStep(g)) {
-        updateAllGrids(g, 0);
-        ++s;
+    const int first = steps > 0 && needsGhostStep(g) ? 1 : 0;
+    const bool pairs = graphable(g) && steps - first >= 2;
+    if (pairs) pairGraph(g, (g->levels[0].info.esotwistFlipper ? 1 : 0) ^ first);  // may fail: before any step
+    try {
+        int s = 0;
+        for (; s < first; ++s) updateAllGrids(g, 0);
+        if (pairs)
+            for (; s + 2 <= steps; s += 2) launchPair(g);
+        for (; s < steps; ++s) updateAllGrids(g, 0);
+    } catch (...) {
+        finishSteps(g);
+        throw;
     }
-    if (graphable(g))
-        for (; s + 2 <= steps; s += 2) launchPair(g);
-    for (; s < steps; ++s) updateAllGrids(g, 0);
     finishSteps(g);
 }
 
@@ -668,8 +673,14 @@ cudaGraphExec_t batchPairGraph(lbm_batch* b, int parity) {
     if (b->pairExec[parity]) return b->pairExec[parity];
     cudaGraph_t graph = nullptr;
     ck(cudaStreamBeginCapture(b->captureStream, cudaStreamCaptureModeThreadLocal), "begin capture");
-    batchStep(b, parity != 0, b->captureStream);
-    batchStep(b, parity == 0, b->captureStream);
+    try {
+        batchStep(b, parity != 0, b->captureStream);
+        batchStep(b, parity == 0, b->captureStream);
+    } catch (...) {
+        cudaStreamEndCapture(b->captureStream, &graph);
+        if (graph) cudaGraphDestroy(graph);
+        throw;
+    }
     const cudaError_t e = cudaStreamEndCapture(b->captureStream, &graph);
     ck(e, "end capture");
     cudaGraphExec_t exec = nullptr;
@@ -681,39 +692,47 @@ cudaGraphExec_t batchPairGraph(lbm_batch* b, int parity) {
 }
 
 // Advance `steps` packed steps on the batch stream (members already waited for).
+// Each step is counted when it is queued, and the members' states are ordinary
+// ones at the end, also of a series that fails.
 void batchAdvance(lbm_batch* b, int steps) {
     if (steps == 0) return;  // the members' states, their ghosts among them, stay as they are
-    bool flip = b->members[0]->levels[0].info.esotwistFlipper;
-    int s = 0;
-    if (!b->wrapped.empty() && capturing(b->stream)) {
-        for (; s < steps; ++s, flip = !flip) batchStep(b, flip, b->stream, GhostCopies::All);
-        for (lbm_grids* g : b->members) {
-            for (int k = 0; k < steps; ++k) advanceHostState(g->levels[0]);
-            g->levels[0].flushPending = false;
+    const bool captured = !b->wrapped.empty() && capturing(b->stream);
+    bool flip = b->members[0]->levels[0].info.esotwistFlipper, stale = false;
+    for (lbm_grids* g : b->wrapped) stale = stale || needsGhostStep(g);
+    const int first = captured ? steps : stale ? 1 : 0;  // steps with ghost copies
+    const bool pairs = graphable(b->members[0]) && steps - first >= 2;
+    if (pairs) batchPairGraph(b, (flip ? 1 : 0) ^ first);  // may fail: before any step
+    auto finish = [&] {
+        for (lbm_grids* g : b->members) finishSteps(g->levels[0], b->stream);
+    };
+    try {
+        int s = 0;
+        for (; s < first; ++s, flip = !flip) {
+            batchStep(b, flip, b->stream, captured ? GhostCopies::All : GhostCopies::Stale);
+            for (lbm_grids* g : b->members) {
+                LevelState& L = g->levels[0];
+                const bool copied = captured || needsGhostStep(g);
+                advanceHostState(L);
+                if (copied) L.flushPending = false;
+                if (!captured) L.ghostsCurrent = true;  // (a capture changes no state)
+            }
         }
-        ck(cudaGetLastError(), "batch launch");
-        return;
+        if (pairs)
+            for (; s + 2 <= steps; s += 2) {
+                ck(cudaGraphLaunch(batchPairGraph(b, flip ? 1 : 0), b->stream), "graph launch");
+                for (lbm_grids* g : b->members)
+                    for (int k = 0; k < 2; ++k) advanceHostState(g->levels[0]);
+            }
+        for (; s < steps; ++s, flip = !flip) {
+            batchStep(b, flip, b->stream);
+            for (lbm_grids* g : b->members) advanceHostState(g->levels[0]);
+        }
+    } catch (...) {
+        finish();
+        cudaStreamSynchronize(b->stream);  // the members' streams are not told to wait
+        throw;
     }
-    for (lbm_grids* g : b->wrapped)
-        if (needsGhostStep(g)) s = 1;
-    if (s == 1) {
-        batchStep(b, flip, b->stream, GhostCopies::Stale);
-        flip = !flip;
-    }
-    if (graphable(b->members[0]))
-        for (; s + 2 <= steps; s += 2) ck(cudaGraphLaunch(batchPairGraph(b, flip ? 1 : 0), b->stream), "graph launch");
-    for (; s < steps; ++s) {
-        batchStep(b, flip, b->stream);
-        flip = !flip;
-    }
-    for (lbm_grids* g : b->members) {
-        LevelState& L = g->levels[0];
-        const bool ghostStep = needsGhostStep(g);
-        for (int k = 0; k < steps; ++k) advanceHostState(L);
-        L.ghostsCurrent = true;
-        if (ghostStep && steps == 1) L.flushPending = false;  // its ghosts were copied
-        finishSteps(L, b->stream);
-    }
+    finish();
     ck(cudaGetLastError(), "batch launch");
 }
 
@@ -1260,24 +1279,40 @@ int lbm_update_batch(lbm_grids* const* grids, int count, int steps) {
     return guarded("lbm_update_batch", [&] {
         // step pairs from each domain's graph, interleaved across domains;
         // domains without graphs (rotors) and a trailing odd step launch directly
-        int s = 0;
-        for (; s + 2 <= steps; s += 2)
-            for (int q = 0; q < count; ++q) {
-                if (capturedWrapped(grids[q])) {
-                    captureSteps(grids[q], 2);
-                } else if (graphable(grids[q]) && !needsGhostStep(grids[q])) {
-                    launchPair(grids[q]);
-                } else {
-                    updateAllGrids(grids[q], 0);
-                    updateAllGrids(grids[q], 0);
+        std::vector<char> captured(count);
+        for (int q = 0; q < count; ++q) {
+            const lbm_grids* g = grids[q];
+            captured[q] = capturedWrapped(g);
+            // may fail: before any step
+            if (graphable(g) && !captured[q] && steps >= (needsGhostStep(g) ? 4 : 2))
+                pairGraph(grids[q], g->levels[0].info.esotwistFlipper ? 1 : 0);
+        }
+        auto finish = [&] {
+            for (int q = 0; q < count; ++q) finishSteps(grids[q]);
+        };
+        try {
+            int s = 0;
+            for (; s + 2 <= steps; s += 2)
+                for (int q = 0; q < count; ++q) {
+                    if (captured[q]) {
+                        captureSteps(grids[q], 2);
+                    } else if (graphable(grids[q]) && !needsGhostStep(grids[q])) {
+                        launchPair(grids[q]);
+                    } else {
+                        updateAllGrids(grids[q], 0);
+                        updateAllGrids(grids[q], 0);
+                    }
                 }
-            }
-        for (; s < steps; ++s)
-            for (int q = 0; q < count; ++q) {
-                if (capturedWrapped(grids[q])) captureSteps(grids[q], 1);
-                else updateAllGrids(grids[q], 0);
-            }
-        for (int q = 0; q < count; ++q) finishSteps(grids[q]);
+            for (; s < steps; ++s)
+                for (int q = 0; q < count; ++q) {
+                    if (captured[q]) captureSteps(grids[q], 1);
+                    else updateAllGrids(grids[q], 0);
+                }
+        } catch (...) {
+            finish();
+            throw;
+        }
+        finish();
         ck(cudaGetLastError(), "step launch");
     });
 }
@@ -1455,6 +1490,7 @@ int lbm_time_steps(lbm_grids* g, int steps, float* ms) {
             if (g->levels[0].dev.wrapped && steps > 0) endLaunches = ghostStep ? (steps > 1) + 1 : 1;
         } catch (...) {
             g->timingKernels = false;
+            finishSteps(g);
             throw;
         }
         g->timingKernels = false;
@@ -1621,6 +1657,7 @@ int lbm_write_f(lbm_grids* g, int level, const float* host, size_t bytes) {
     const size_t need = 27ULL * L.dev.cellCount * 4;
     if (bytes != need) return fail(LBM_ERR_INVALID, "lbm_write_f: byte count does not match");
     return guarded("lbm_write_f", [&] {
+        g->levels[0].ghostsCurrent = false;  // also when the copy ends half way
         copyPopulations<false>(g, L, host);
         checkGhosts(g);
     });
@@ -2081,6 +2118,7 @@ int lbm_load_state(lbm_grids* g, const void* host, size_t bytes) {
     }
     return guarded("lbm_load_state", [&] {
         const unsigned char* p = in + 16;
+        g->levels[0].ghostsCurrent = false;  // also when the copy ends half way
         for (LevelState& L : g->levels) {
             StateHeader h;
             std::memcpy(&h, p, sizeof(h));

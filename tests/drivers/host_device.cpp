@@ -44,7 +44,7 @@ std::recursive_mutex lock;
 std::map<const void*, Model> models;
 std::map<cudaStream_t, Stream> streams;
 bool initialGhosts = true;
-int launches = 0, instantiateLeft = -1, copyDelayUs = 0;
+int launches = 0, instantiateLeft = -1, uploadsLeft = -1, copyDelayUs = 0;
 size_t pitchLimit = 0x7fffffff;
 
 cudaError_t run(cudaStream_t s, std::function<void()> op) {
@@ -74,13 +74,14 @@ void host_device_reset(int ghosts) {
     streams.clear();
     initialGhosts = ghosts != 0;
     launches = 0;
-    instantiateLeft = -1;
+    instantiateLeft = uploadsLeft = -1;
     copyDelayUs = 0;
     pitchLimit = 0x7fffffff;
 }
 int host_device_launches() { return launches; }
-// graph instantiations that succeed from now on (-1: all)
+// graph instantiations and copies to the device that succeed from now on (-1: all)
 void host_device_instantiations(int n) { instantiateLeft = n; }
+void host_device_uploads(int n) { uploadsLeft = n; }
 void host_device_copy_delay(int us) { copyDelayUs = us; }
 void host_device_pitch_limit(size_t bytes) { pitchLimit = bytes; }
 // {steps, ghosts, due, wrong} of the order-th level built
@@ -156,6 +157,8 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t s) {
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t s) { return run(s, [=] { std::memset(p, v, n); }); }
 cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t n, cudaMemcpyKind kind, cudaStream_t s) {
     if (kind == cudaMemcpyDeviceToHost && copyDelayUs) usleep(copyDelayUs);
+    if (kind == cudaMemcpyHostToDevice && uploadsLeft == 0) return cudaErrorUnknown;
+    if (kind == cudaMemcpyHostToDevice && uploadsLeft > 0) --uploadsLeft;
     return run(s, [=] { std::memcpy(to, from, n); });
 }
 cudaError_t cudaMemcpy2DAsync(void* to, size_t toPitch, const void* from, size_t fromPitch, size_t width, size_t rows,

@@ -162,3 +162,60 @@ def test_fields_wider_than_a_pitched_copy(device):
         assert m[0].nbytes > 1 << 20
         cells = np.arange(m.shape[1], dtype=np.float32) * 16
         np.testing.assert_array_equal(m, cells + 4 * np.arange(4, dtype=np.float32)[:, None])
+
+
+@pytest.mark.parametrize("ghosts", [False, True])
+@pytest.mark.parametrize("graphs", [0, 1, 2])
+@pytest.mark.parametrize("call", ["single", "update_batch", "packed"])
+def test_a_failed_call_leaves_ordinary_states(device, call, graphs, ghosts):
+    """The runtime refuses a graph in the middle of a call: the steps that ran
+    are counted, and every domain is left in a state that readers may use."""
+    lib = device(ghosts)
+    # the last one steps without graphs, and is therefore stepped in any case
+    grids = [L.build_grids(L.periodic_box(6, 4, 4 + 2 * q)) for q in range(3)]
+    grids[2].set_graphs(call == "packed")
+    batch = L.PackedBatch(grids) if call == "packed" else None
+    lib.host_device_instantiations(graphs)
+
+    def advance(n):
+        try:
+            if batch:
+                batch.update(n)
+            elif call == "update_batch":
+                L.update_batch([grids[2], *grids[:2]], n)
+            else:
+                for g in grids:
+                    g.update_all_grids(n)
+        except A.LbmError:
+            return False
+        return True
+
+    enough = {"single": 2, "update_batch": 2, "packed": 1}[call]
+    assert advance(7) == (graphs >= enough)
+    for q, g in enumerate(grids):
+        assert level(lib, q) == {**done(g.info().iterations_finished), "ghosts": level(lib, q)["ghosts"]}
+        g.macro()
+    lib.host_device_instantiations(-1)
+    before = [g.info().iterations_finished for g in grids]
+    if batch:
+        assert len(set(before)) == 1
+    assert advance(5)
+    for q, g in enumerate(grids):
+        assert level(lib, q) == done(before[q] + 5)
+    if batch:
+        batch.close()
+    for g in grids:
+        g.close()
+
+
+def test_a_failed_write_leaves_ghosts_unknown(device):
+    """Populations written in part: the next step copies the ghosts."""
+    lib = device(True)
+    with L.build_grids(L.periodic_box(64, 64, 64)) as g:
+        f = g.populations()
+        lib.host_device_uploads(3)
+        with pytest.raises(A.LbmError):
+            g.set_populations(f)
+        lib.host_device_uploads(-1)
+        g.update_all_grids(2)
+        assert level(lib) == done(2)
