@@ -385,7 +385,10 @@ typedef struct lbm_batch_info {
     int open_chunks;          /* open-boundary CTAs per step                  */
     int periodic_cells;       /* periodic ghost cells of all members          */
     int launches_per_step;    /* kernels one packed step launches: up to 3, and
-                                 one per 16 members that are periodic boxes   */
+                                 one per 16 members that are periodic boxes;
+                                 a call ends with one more per 16 of those, and
+                                 its first step takes two more when ghosts of
+                                 theirs differ from their sources             */
 } lbm_batch_info;
 int lbm_batch_create(lbm_grids* const* grids, int count, lbm_batch** out);
 int lbm_batch_update(lbm_batch* b, int coarse_steps);

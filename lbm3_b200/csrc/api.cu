@@ -316,7 +316,8 @@ void updateSingleGrid(lbm_grids* g, LevelState& L, cudaStream_t stream) {
 // wrapped level, on the stream its last step ran on.
 void finishSteps(LevelState& L, cudaStream_t stream) {
     if (!L.flushPending) return;
-    lbm::launchWrappedFlush(L.dev, L.info.esotwistFlipper, stream);
+    const lbm::DevLevel* level = &L.dev;
+    lbm::launchWrappedFlush(&level, 1, L.info.esotwistFlipper, stream);
     L.flushPending = false;
 }
 void finishSteps(lbm_grids* g) {
@@ -622,6 +623,8 @@ struct lbm_batch {
     std::vector<lbm_grids*> wrapped;  // the members that step without ghosts, outside the packed tables
     int storage = LBM_STORE_F32;
     lbm::DevBatch dev{};
+    lbm::DevBatch ghostDev{};  // packed tables of the wrapped members, for steps with ghost copies
+    int* staleItems = nullptr; // room for ghostDev's itemStart and periodicStart of some of them
     lbm_batch_info info{};
     std::vector<void*> owned;
     cudaStream_t stream = nullptr;         // the batch's launches
@@ -650,20 +653,32 @@ namespace {
 enum class GhostCopies { None, Stale, All };
 
 // One step of all members: the packed launches, and the ghost-free ones of the
-// dense periodic members.  A member that copies ghosts (never inside a graph of
-// the batch) steps on its own through the packed kernel as a batch of one, so
-// that what it computes does not depend on the other members.
+// dense periodic members.  Members that copy ghosts (never inside a graph of the
+// batch) step through the packed kernels too, in which what a member computes
+// does not depend on the others.
 void batchStep(lbm_batch* b, bool flip, cudaStream_t s, GhostCopies copies = GhostCopies::None) {
     if (b->dev.domainCount > 0) lbm::launchPackedStep(b->dev, b->storage, flip, s);
     std::vector<const lbm::DevLevel*> levels;
+    // prefix sums of the items and of the ghosts, the other members without any
+    std::vector<int> start(1, 0), ghosts(1, 0);
     for (lbm_grids* g : b->wrapped) {
         LevelState& L = g->levels[0];
-        if (copies == GhostCopies::All || (copies == GhostCopies::Stale && !L.ghostsCurrent)) {
-            lbm::launchCollidePacked(L.dev, flip, s);
-            lbm::launchPeriodic(L.dev, !flip, s);
-        } else {
-            levels.push_back(&L.dev);
-        }
+        const bool copy = copies == GhostCopies::All || (copies == GhostCopies::Stale && !L.ghostsCurrent);
+        if (!copy) levels.push_back(&L.dev);
+        start.push_back(start.back() + (copy ? lbm::pairItems(L.dev) : 0));
+        ghosts.push_back(ghosts.back() + (copy ? L.dev.perCount : 0));
+    }
+    if (levels.empty() && !b->wrapped.empty()) {
+        lbm::launchPackedStep(b->ghostDev, b->storage, flip, s);
+    } else if (start.back() > 0) {
+        lbm::DevBatch some = b->ghostDev;
+        some.itemStart = b->staleItems;
+        some.collideCount = start.back();
+        some.periodicStart = b->staleItems + start.size();
+        some.periodicCount = ghosts.back();
+        start.insert(start.end(), ghosts.begin(), ghosts.end());
+        ck(cudaMemcpyAsync(b->staleItems, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice, s), "copy");
+        lbm::launchPackedStep(some, b->storage, flip, s);
     }
     lbm::launchWrapped(levels.data(), static_cast<int>(levels.size()), flip, s);
 }
@@ -703,7 +718,13 @@ void batchAdvance(lbm_batch* b, int steps) {
     const bool pairs = graphable(b->members[0]) && steps - first >= 2;
     if (pairs) batchPairGraph(b, (flip ? 1 : 0) ^ first);  // may fail: before any step
     auto finish = [&] {
-        for (lbm_grids* g : b->members) finishSteps(g->levels[0], b->stream);
+        std::vector<const lbm::DevLevel*> due;
+        for (lbm_grids* g : b->wrapped) {
+            if (g->levels[0].flushPending) due.push_back(&g->levels[0].dev);
+            g->levels[0].flushPending = false;
+        }
+        lbm::launchWrappedFlush(due.data(), static_cast<int>(due.size()),
+                                b->members[0]->levels[0].info.esotwistFlipper, b->stream);
     };
     try {
         int s = 0;
@@ -1337,47 +1358,57 @@ int lbm_batch_create(lbm_grids* const* grids, int count, lbm_batch** out) {
             if (b->storage == LBM_STORE_F64) throw std::invalid_argument("FP64 domains are not packed");
             if (!lbm::pairFits(L.dev)) throw std::invalid_argument("a member is too large for 32-bit offsets");
         }
-        // packed tables: every member's items, member by member
-        std::vector<lbm::DevLevel> levels;
-        std::vector<int2> open;
-        std::vector<int> itemStart{0};
-        std::vector<int> perStart{0};
-        long long cells = 0;
-        int ghosts = 0, items = 0;
-        for (lbm_grids* g : b->members) {
-            const lbm::DevLevel& d = g->levels[0].dev;
-            cells += d.cellCount;
-            ghosts += d.perCount;
-            items += lbm::pairItems(d);
-            if (d.wrapped) {
-                b->wrapped.push_back(g);
-                continue;
-            }
-            const int q = static_cast<int>(levels.size());
-            levels.push_back(d);
-            itemStart.push_back(itemStart.back() + lbm::pairItems(d));
-            for (int i = 0; i < d.obChunkCount; ++i) open.push_back(make_int2(q, i));
-            perStart.push_back(perStart.back() + d.perCount);
-        }
-        const int packed = static_cast<int>(levels.size());
         ck(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "stream");
         ck(cudaStreamCreateWithFlags(&b->captureStream, cudaStreamNonBlocking), "stream");
         ck(cudaEventCreateWithFlags(&b->sync, cudaEventDisableTiming), "event");
         ck(cudaEventCreate(&b->ev0), "event");
         ck(cudaEventCreate(&b->ev1), "event");
         auto own = [&](auto* p) { if (p) b->owned.push_back(p); return p; };
-        lbm::DevBatch& D = b->dev;
-        D.levels = own(upload(levels, b->stream));
-        D.domainCount = packed;
-        D.itemStart = own(upload(itemStart, b->stream));
-        D.collideCount = itemStart.back();
-        D.work = own(devAlloc<int>(packed + 1));
-        ck(cudaMemsetAsync(D.work, 0, (packed + 1) * sizeof(int), b->stream), "memset");
-        D.openItems = open.empty() ? nullptr : own(upload(open, b->stream));
-        D.openCount = static_cast<int>(open.size());
-        D.periodicStart = own(upload(perStart, b->stream));
-        D.periodicCount = perStart.back();
-        ck(cudaStreamSynchronize(b->stream), "batch upload");
+        long long cells = 0;
+        int ghosts = 0, items = 0;
+        std::vector<lbm_grids*> packed;
+        for (lbm_grids* g : b->members) {
+            const lbm::DevLevel& d = g->levels[0].dev;
+            cells += d.cellCount;
+            ghosts += d.perCount;
+            items += lbm::pairItems(d);
+            (d.wrapped ? b->wrapped : packed).push_back(g);
+        }
+        // packed tables: every member's items, member by member
+        auto tables = [&](const std::vector<lbm_grids*>& members) {
+            std::vector<lbm::DevLevel> levels;
+            std::vector<int2> open;
+            std::vector<int> itemStart{0};
+            std::vector<int> perStart{0};
+            for (lbm_grids* g : members) {
+                const lbm::DevLevel& d = g->levels[0].dev;
+                const int q = static_cast<int>(levels.size());
+                levels.push_back(d);
+                itemStart.push_back(itemStart.back() + lbm::pairItems(d));
+                for (int i = 0; i < d.obChunkCount; ++i) open.push_back(make_int2(q, i));
+                perStart.push_back(perStart.back() + d.perCount);
+            }
+            const int count = static_cast<int>(levels.size());
+            lbm::DevBatch D{};
+            D.levels = own(upload(levels, b->stream));
+            D.domainCount = count;
+            D.itemStart = own(upload(itemStart, b->stream));
+            D.collideCount = itemStart.back();
+            D.work = own(devAlloc<int>(count + 1));
+            ck(cudaMemsetAsync(D.work, 0, (count + 1) * sizeof(int), b->stream), "memset");
+            D.openItems = open.empty() ? nullptr : own(upload(open, b->stream));
+            D.openCount = static_cast<int>(open.size());
+            D.periodicStart = own(upload(perStart, b->stream));
+            D.periodicCount = perStart.back();
+            ck(cudaStreamSynchronize(b->stream), "batch upload");
+            return D;
+        };
+        if (!packed.empty()) b->dev = tables(packed);
+        if (!b->wrapped.empty()) {
+            b->ghostDev = tables(b->wrapped);
+            b->staleItems = own(devAlloc<int>(2 * (b->wrapped.size() + 1)));
+        }
+        const lbm::DevBatch& D = b->dev;
         b->info.domain_count = count;
         b->info.cells = cells;
         b->info.collide_items = items;

@@ -147,6 +147,10 @@ constexpr int kWrapDomains = 16;
 template <class T> struct WrapBatch {
     WrapDomain<T> dom[kWrapDomains];
 };
+// Their descriptors on the device (DevLevel::self), for the ghost exchange.
+struct FlushBatch {
+    const DevLevel* level[kWrapDomains];
+};
 
 // One level's pass over the section image of a flow report
 // (getFlowReportGeneral, include/flowReportFunctions.h:96-262): the cells of

@@ -40,9 +40,6 @@ void launchCollideStream(const DevLevel& g, bool flip, cudaStream_t s) {
                         paired && (!pairFits(g) || g.storage == LBM_STORE_F64) ? CollideVariant::Prefetch : v)
     }
 }
-void launchCollidePacked(const DevLevel& g, bool flip, cudaStream_t s) {
-    LBM3_BY_STORAGE(launchCollidePair, g, flip, s)
-}
 void launchRotorCells(const DevLevel& g, bool flip, cudaStream_t s) {
     LBM3_BY_STORAGE(launchRotorCells, g, flip, s)
 }
@@ -51,8 +48,10 @@ void launchWrapped(const DevLevel* const* levels, int count, bool flip, cudaStre
     const DevLevel& g = *levels[0];
     LBM3_BY_STORAGE(launchWrapped, levels, count, flip, s)
 }
-void launchWrappedFlush(const DevLevel& g, bool flip, cudaStream_t s) {
-    LBM3_BY_STORAGE(launchWrappedFlush, g, flip, s)
+void launchWrappedFlush(const DevLevel* const* levels, int count, bool flip, cudaStream_t s) {
+    if (count <= 0) return;
+    const DevLevel& g = *levels[0];
+    LBM3_BY_STORAGE(launchWrappedFlush, levels, count, flip, s)
 }
 void launchGhostsDiffer(const DevLevel& g, bool flip, cudaStream_t s, int* differ) {
     LBM3_BY_STORAGE(launchGhostsDiffer, g, flip, s, differ)

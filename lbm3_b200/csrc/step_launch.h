@@ -60,15 +60,13 @@ void launchPackedStep(const DevBatch& b, int storage, bool flip, cudaStream_t s)
 // restores the ordinary state after the last of a series of such steps
 // (flip: the flipper after streaming).
 void launchWrapped(const DevLevel* const* levels, int count, bool flip, cudaStream_t s);
-void launchWrappedFlush(const DevLevel& g, bool flip, cudaStream_t s);
+void launchWrappedFlush(const DevLevel* const* levels, int count, bool flip, cudaStream_t s);
 // sets *differ (a device word that holds 0) when a ghost's values are not its
 // source's; only on a state whose ghosts all agree may wrapped steps start
 void launchGhostsDiffer(const DevLevel& g, bool flip, cudaStream_t s, int* differ);
 inline int wrappedLaunches(int count) { return (count + kWrapDomains - 1) / kWrapDomains; }
 // rotor cells of a level (part of launchCollideStream, separate for wrapped levels)
 void launchRotorCells(const DevLevel& g, bool flip, cudaStream_t s);
-// collide-stream of one level through the packed kernel (a batch of one)
-void launchCollidePacked(const DevLevel& g, bool flip, cudaStream_t s);
 
 // per-storage launchers (one set per step.cu unit)
 #define LBM3_DECLARE_STORAGE_LAUNCHERS(SUF)                                                                      \
@@ -89,7 +87,7 @@ void launchCollidePacked(const DevLevel& g, bool flip, cudaStream_t s);
                                int h1, int v0, int v1, double* out);                                           \
     void launchPackedStep##SUF(const DevBatch& b, bool flip, cudaStream_t s);                                   \
     void launchWrapped##SUF(const DevLevel* const* levels, int count, bool flip, cudaStream_t s);              \
-    void launchWrappedFlush##SUF(const DevLevel& g, bool flip, cudaStream_t s);                                \
+    void launchWrappedFlush##SUF(const DevLevel* const* levels, int count, bool flip, cudaStream_t s);         \
     void launchGhostsDiffer##SUF(const DevLevel& g, bool flip, cudaStream_t s, int* differ);                  \
     void launchRotorCells##SUF(const DevLevel& g, bool flip, cudaStream_t s);                                  \
     void launchFlowImage##SUF(const DevLevel& g, bool flip, cudaStream_t s, const FlowImagePass& a, float* img);

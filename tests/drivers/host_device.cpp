@@ -182,7 +182,6 @@ void launchInit(const DevLevel& g, bool, cudaStream_t, const float4*, float4) {
 }
 void launchOpenBoundaryInit(const DevLevel&, bool, cudaStream_t) {}
 void launchCollideStream(const DevLevel& g, bool, cudaStream_t s) { launch(s, [&m = of(g)] { collide(m); }); }
-void launchCollidePacked(const DevLevel& g, bool, cudaStream_t s) { launch(s, [&m = of(g)] { collide(m); }); }
 void launchPeriodic(const DevLevel& g, bool, cudaStream_t s) { launch(s, [&m = of(g)] { copyGhosts(m); }); }
 void launchRotorCells(const DevLevel&, bool, cudaStream_t) {}
 void launchOpenBoundary(const DevLevel&, bool, cudaStream_t) {}
@@ -199,7 +198,15 @@ void launchWrapped(const DevLevel* const* levels, int count, bool, cudaStream_t 
         });
     }
 }
-void launchWrappedFlush(const DevLevel& g, bool, cudaStream_t s) { launch(s, [&m = of(g)] { m.due = false; }); }
+void launchWrappedFlush(const DevLevel* const* levels, int count, bool, cudaStream_t s) {
+    for (int first = 0; first < count; first += kWrapDomains) {
+        std::vector<Model*> flush;
+        for (int q = first; q < std::min(count, first + kWrapDomains); ++q) flush.push_back(&of(*levels[q]));
+        launch(s, [flush] {
+            for (Model* m : flush) m->due = false;
+        });
+    }
+}
 void launchGhostsDiffer(const DevLevel& g, bool, cudaStream_t s, int* differ) {
     launch(s, [&m = of(g), differ] { reads(m); *differ = !m.ghosts; });
 }

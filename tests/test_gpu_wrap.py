@@ -133,3 +133,28 @@ def test_batch_timed_over_no_steps():
         e_rho, e_u, _ = density_velocity_errors(g.macro(), o.macro())
         assert e_rho < FIELD_REL_L2 and e_u < FIELD_REL_L2, (e_rho, e_u)
     o.close()
+
+
+@pytest.mark.parametrize("storage", [A.LBM_STORE_F32, A.LBM_STORE_BF16])
+def test_batch_with_one_written_member(storage):
+    """Only the written member's ghosts differ: it steps with ghost copies, the
+    others without, and each ends where it ends as a batch of its own."""
+    cases = [_case((6 + 2 * q, 8, 4), storage) for q in range(3)]
+
+    def run(grids, which):
+        with L.PackedBatch(grids) as b:
+            b.update(2)
+            for q, g in zip(which, grids):
+                if q == 1:
+                    f = g.populations()
+                    g.set_populations(f * (1 + 1e-2 * np.random.default_rng(6).standard_normal(f.shape).astype(np.float32)))
+            for steps in (1, 1, 3):
+                b.update(steps)
+        return [g.populations() for g in grids]
+    grids = [L.build_grids(c) for c in cases]
+    together = run(grids, range(3))
+    for q, c in enumerate(cases):
+        with L.build_grids(c) as alone:
+            np.testing.assert_array_equal(run([alone], [q])[0], together[q])
+    for g in grids:
+        g.close()

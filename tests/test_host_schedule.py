@@ -219,3 +219,23 @@ def test_a_failed_write_leaves_ghosts_unknown(device):
         lib.host_device_uploads(-1)
         g.update_all_grids(2)
         assert level(lib) == done(2)
+
+
+@pytest.mark.parametrize("stale", [0, 1, 20])
+def test_launches_of_a_one_step_batch_call(device, stale):
+    """A packed batch of 20 periodic boxes, one step per call: two launches for
+    the step (16 domains each) and two for the ghost exchange; two (collision
+    and ghost copies) for the members with new populations, however many."""
+    lib = device(True)
+    grids = [L.build_grids(L.periodic_box(4, 4, 4)) for _ in range(20)]
+    with L.PackedBatch(grids) as b:
+        for n, changed in enumerate((0, stale, 0)):
+            for g in grids[:changed]:
+                g.set_populations(g.populations())
+            before = lib.host_device_launches()
+            b.update(1)
+            fresh = 20 - changed
+            assert lib.host_device_launches() - before == 2 * -(-fresh // 16) + (2 if changed else 0)
+            assert [level(lib, q) for q in range(20)] == [done(n + 1)] * 20
+    for g in grids:
+        g.close()
