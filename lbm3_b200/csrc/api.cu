@@ -331,7 +331,7 @@ bool needsGhostStep(const lbm_grids* g) {
 }
 
 // After the populations were set from outside: see whether the ghosts repeat
-// their sources.  The stream is idle afterwards.
+// their sources (the stream is idle afterwards where it had to look).
 void checkGhosts(lbm_grids* g) {
     LevelState& L = g->levels[0];
     L.flushPending = false;
@@ -1256,8 +1256,8 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out, long long* fluidUpdates)
             L.dev.self = self;
             ck(cudaMemcpyAsync(self, &L.dev, sizeof(lbm::DevLevel), cudaMemcpyHostToDevice, s), "descriptor copy");
         }
-        ck(cudaStreamSynchronize(s), "build sync");
         checkGhosts(g);
+        ck(cudaStreamSynchronize(s), "build sync");
         if (fluidUpdates) *fluidUpdates = host.fluidUpdatesPerIteration;
         // the driver's hooks are evaluated during the build only
         g->c.open_bc_hook = nullptr;

@@ -995,11 +995,12 @@ bool ghostFreePeriodic(const HostLevel& L, std::vector<uint32_t>& skip) {
     if (in.gridID != 0 || mx < 2 || my < 2 || mz < 2 || n != nx * ny * nz) return false;
     if (!L.openCells.empty() || !L.wallIndex.empty() || L.wallCellCount != 0) return false;
     if (static_cast<long long>(L.perIndex.size()) != n - mx * my * mz) return false;
+    auto inside = [](long long v, long long m) { return v == 0 ? m : v == m + 1 ? 1 : v; };
     for (size_t q = 0; q < L.perIndex.size(); ++q) {
         const int c = L.perIndex[q];
-        auto inside = [](long long v, long long m) { return v == 0 ? m : v == m + 1 ? 1 : v; };
-        const long long i = inside(c % nx, mx), j = inside(c / nx % ny, my), k = inside(c / (nx * ny), mz);
-        if (L.perSource[q] != i + nx * (j + ny * k)) return false;
+        const long long i = L.I[c], j = L.J[c], k = L.K[c];
+        if (c != i + nx * (j + ny * k)) return false;
+        if (L.perSource[q] != inside(i, mx) + nx * (inside(j, my) + ny * inside(k, mz))) return false;
     }
     if (L.rotorCells.empty()) return true;
     skip.assign(static_cast<size_t>((mx * my * mz + 31) / 32), 0u);
