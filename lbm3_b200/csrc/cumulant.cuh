@@ -52,7 +52,6 @@ template <class T> struct CollisionConstsT {
     T halfW1c;     // 1 - 0.5 * omega1
     T oneMinusW3, oneMinusW4, oneMinusW5;
     T c43;         // (2/3) * tauTerm * A
-    T c45;         // -(4/3) * tauTerm * A
     T cB;          // -(1/3) * tauTerm * B
 };
 using CollisionConsts = CollisionConstsT<float>;
@@ -95,7 +94,6 @@ template <class T> inline CollisionConstsT<T> makeCollisionConstsT(T nu, T nuMul
     k.oneMinusW4 = T(1) - k.omega4;
     k.oneMinusW5 = T(1) - k.omega5;
     k.c43 = (T(2) / T(3)) * k.tauTerm * k.A;
-    k.c45 = -(T(4) / T(3)) * k.tauTerm * k.A;
     k.cB = -(T(1) / T(3)) * k.tauTerm * k.B;
     return k;
 }
@@ -415,9 +413,10 @@ LBM_HD void collideCumulantT(R (&f)[27], const CollisionConstsT<typename ScalarO
         Cs201 = e119 + e122;
         Cs021 = e119 - e122;
         Cs111 = relax(P.oneMinusW5, C111);
-        // fourth order (:310-323): with e45 = -2 (2/3) tau A rho (Dxu + Dyv + Dzw)
-        // the combinations reduce to two strain rates each, and rho times the
-        // shear rates to the moments they came from
+        // fourth order (:310-323): omega6 = omega7 = 1 make the coefficient of the
+        // trace, e45 = -(4/3) tau A rho (Dxu + Dyv + Dzw), minus twice that of
+        // e43 and e44, c43 rho: the combinations reduce to two strain rates
+        // each, and rho times the shear rates to the moments they came from
         const R mrc43 = rho * -P.c43;
         f220 = fmaR(mrc43, Dxu + Dyv, f220);
         f202 = fmaR(mrc43, Dxu + Dzw, f202);
@@ -519,10 +518,6 @@ LBM_HD void collideCumulantT(R (&f)[27], const CollisionConstsT<typename ScalarO
                     f[dirOf(a - 1, b - 1, 0)], f[dirOf(a - 1, b - 1, 1)]);
             }
     }
-}
-
-LBM_HD void collideCumulant(float (&f)[27], const CollisionConsts& P, float lambda, float gx, float gy, float gz) {
-    collideCumulantT<float>(f, P, lambda, gx, gy, gz);
 }
 
 }  // namespace lbm
