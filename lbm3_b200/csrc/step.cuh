@@ -128,8 +128,10 @@ struct DevBatch {
 
 // A dense periodic level as the ghost-free step sees it (stepWrapped in
 // step.cu): nx x ny x nz cells of which the outermost layer are periodic
-// ghosts; T is the arithmetic type.  Passed by value.
-template <class T> struct WrapDomain {
+// ghosts; T is the arithmetic type.  Passed by value, 16-byte aligned so that its
+// constants can be loaded in wide pieces (160^3 FP16 146.0 us per step, 146.8
+// with the natural 8 bytes).
+template <class T> struct alignas(16) WrapDomain {
     void* f;                  // populations [27][stride]
     unsigned* seed;           // as DevLevel::seed
     const unsigned* skip;     // one bit per interior cell that another kernel collides; null: none
