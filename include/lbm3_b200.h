@@ -341,7 +341,9 @@ int lbm_build_grids(const lbm_case* c, lbm_grids** out,
 void lbm_free_grids(lbm_grids* g);
 
 /* Launch subsequent work on this CUDA stream (cudaStream_t passed as void*,
- * NULL = legacy default stream). */
+ * NULL = legacy default stream).  A program may capture steps on it into a graph
+ * of its own: one step per lbm_update_all_grids call, and an even number in all,
+ * so that every replay finds the state at the captured parity. */
 int lbm_set_stream(lbm_grids* g, void* stream);
 
 /* Advance `coarse_steps` coarse time steps (asynchronous on the grid stream).
@@ -360,13 +362,15 @@ int lbm_update_all_grids(lbm_grids* g, int coarse_steps);
 int lbm_update_batch(lbm_grids* const* grids, int count, int coarse_steps);
 
 /* Packed batch: single-level domains (without rotors, of one storage type,
- * FP32, FP16 or BF16) advanced by ONE persistent collide-stream launch over a
- * packed table of all domains' work items (per domain its listed-cell chunks
- * and 128-cell bulk tiles, with an item counter each: a CTA works through its
- * home domain, then helps the others), one open-boundary launch over all
- * domains' chunks
- * and one periodic-ghost launch, instead of a launch set per domain; step
- * pairs replay as a CUDA graph.  A member's result is bit-identical to the
+ * FP32, FP16 or BF16) advanced by a few launches per step instead of a launch
+ * set per domain.  Periodic boxes (dense, ghosts on every face, no walls) step
+ * without ghosts, 16 of them per launch.  All other members take ONE persistent
+ * collide-stream launch over a packed table of their work items (per domain its
+ * listed-cell chunks and 128-cell bulk tiles, with an item counter each: a CTA
+ * works through its home domain, then helps the others), one open-boundary
+ * launch over all their chunks and one periodic-ghost launch; boxes whose ghosts
+ * differ from their sources (new populations) do so too, in a call's first step.
+ * Step pairs replay as a CUDA graph.  A member's result is bit-identical to the
  * member stepped as a batch of one (the per-item work does not depend on the
  * other members) and agrees to FP32 rounding with lbm_update_all_grids, whose
  * kernel takes the level descriptor as a kernel parameter.  The batch runs on its own stream, ordered after the
@@ -381,7 +385,9 @@ typedef struct lbm_batch lbm_batch;
 typedef struct lbm_batch_info {
     int domain_count;
     long long cells;          /* sum of the members' cells (ghosts included) */
-    int collide_items;        /* collide-stream work items of all members     */
+    int collide_items;        /* work items of all members in the packed tables
+                                 (boxes included, which take theirs only in a
+                                 step with ghost copies)                      */
     int open_chunks;          /* open-boundary CTAs per step                  */
     int periodic_cells;       /* periodic ghost cells of all members          */
     int launches_per_step;    /* kernels one packed step launches: up to 3, and

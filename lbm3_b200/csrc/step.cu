@@ -1736,8 +1736,8 @@ __global__ void __launch_bounds__(kBlock) scatterF(DevLevel g, long long first, 
 // Cell-wise collision of a batch: two cells per thread with the packed
 // arithmetic, cells t and t + kHalf of a 128-cell tile, so both are coalesced
 // at any batch size and share their plane addresses.  Bound by memory (216
-// bytes per cell): 34 us for 1,000,003 cells, 97% of the copy bandwidth; one
-// cell per thread took 47 us.
+// bytes per cell): 1,000,003 cells take 39 us from HBM, 84% of the copy bandwidth,
+// and 35 when they are partly in the L2 cache; one cell per thread took 53 and 49.
 __global__ void __launch_bounds__(kHalf, LBM3_PAIR_MIN_BLOCKS) collideBatch(float* f, int n, CollisionConsts P,
                                                                           float gx, float gy, float gz) {
     const unsigned t = threadIdx.x;
@@ -1900,9 +1900,9 @@ __global__ void __launch_bounds__(kBlock) periodicPacked(DevBatch b) {
 // parameters, and with them every plane base, to be uniform.
 //
 // Step of a Taylor-Green box, collide-stream and ghost copy before, this kernel
-// now: 64^3 FP32 20.4 -> 10.8 us, 64^3 FP64 45 -> 18.5, 128^3 FP32 112 -> 79,
-// 160^3 FP16 189 -> 147, eight 64^3 FP16 137 -> 77.  FP32 and FP64 are bound by
-// memory (87% of the copy bandwidth at 128^3), FP16 by instruction issue (62% of
+// now: 64^3 FP32 20.4 -> 10.8 us, 64^3 FP64 45 -> 18.5, 128^3 FP32 112 -> 75.5,
+// 160^3 FP16 189 -> 146, eight 64^3 FP16 137 -> 77.  FP32 and FP64 are bound by
+// memory (92% of the copy bandwidth at 128^3), FP16 by instruction issue (62% of
 // the slots, the FMA pipe 55% and the ALU pipe 47% active).
 // Ten or more CTAs of 64 threads per SM (96 registers and less) spill: 107 us
 // at 128^3.

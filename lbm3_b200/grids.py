@@ -345,10 +345,10 @@ def update_batch(grids, coarse_steps: int = 1):
 
 
 class PackedBatch:
-    """Single-level domains advanced by one packed launch per kernel kind
-    (lbm_batch_create): one persistent collide-stream over the packed
-    {domain, item} table of all members, one open-boundary and one
-    periodic-ghost launch; each member's result is bit-identical to the member
+    """Single-level domains advanced together (lbm_batch_create): periodic boxes
+    by one launch of the ghost-free step per 16 of them, all other members by
+    one persistent collide-stream over their packed {domain, item} table, one
+    open-boundary and one periodic-ghost launch; each member's result is bit-identical to the member
     run as a batch of one and agrees to FP32 rounding with update_all_grids.
     Free (close) the batch before its members."""
 

@@ -10,7 +10,8 @@ Active domains keep their populations and tables resident and advance in
 chunks of steps.  Single-level domains without rotors advance in a packed
 batch per storage type: one persistent collide-stream launch over the packed
 block table of all of them, one open-boundary and one periodic launch per
-step, replayed as a CUDA graph (PackedBatch); the batch is rebuilt whenever
+step (periodic boxes: one launch per 16), replayed as a CUDA graph
+(PackedBatch); the batch is rebuilt whenever
 a domain joins or leaves.  A domain that joins at the other esotwist parity
 than the batch steps once on its own first (as a batch of one).  Other domains (several levels,
 rotors, FP64) advance with update_batch on their own streams.  A finished
@@ -18,7 +19,7 @@ domain reads its result, frees its memory and its slot, and the next
 waiting request is admitted.
 
 Each result is the one the request gets when served alone: a packable
-domain always steps through the packed kernel (alone it is a batch of one),
+domain always steps through the batch's kernels (alone it is a batch of one),
 whose per-item work does not depend on the other members, so its fields are
 bit-identical alone and in the mix; against lbm_update_all_grids, whose
 kernel takes the level descriptor as a parameter, they agree to FP32
