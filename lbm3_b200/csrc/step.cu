@@ -644,38 +644,44 @@ template <class T, int N> struct SpecialScratch {
 // Weights of the interpolated bounceback by packed link code c (gamma = c / 254
 // within [0.01, 1]): (1 - gamma) / (1 + gamma) of the pre-collision value,
 // gamma / (1 + gamma) of the two collided ones, 1 / (1 + gamma) of the wall
-// term, evaluated in FP32 as the formula stands.  A table, because two
-// divisions per link are half of a wall-adjacent cell's arithmetic.
-struct alignas(16) LinkWeights {
-    float v[256][4];
+// term, evaluated in T as the formula stands.  A table, because two divisions
+// per link are half of a wall-adjacent cell's arithmetic (FP64 step of a
+// 40x20x20 box with a body, interpolated 21.4 -> 15.3 us, halfway 20.5 -> 14.4;
+// with a branch per link in place of straight-line code 24.9 and 19.1).
+template <class T> struct alignas(16) LinkWeights {
+    T v[256][4];
     constexpr LinkWeights() : v{} {
         for (int c = 0; c < 256; ++c) {
-            const float q = static_cast<float>(c) / 254.f;
-            const float gamma = q < 0.01f ? 0.01f : q > 1.f ? 1.f : q;
-            const float invDen = 1.f / (1.f + gamma);
-            v[c][0] = (1.f - gamma) * invDen;
+            const T q = static_cast<T>(c) / T(254);
+            const T gamma = q < T(0.01f) ? T(0.01f) : q > T(1) ? T(1) : q;
+            const T invDen = T(1) / (T(1) + gamma);
+            v[c][0] = (T(1) - gamma) * invDen;
             v[c][1] = gamma * invDen;
             v[c][2] = invDen;
-            v[c][3] = 0.f;
+            v[c][3] = T(0);
         }
     }
 };
-__device__ const LinkWeights kLinkWeights = LinkWeights();
+__device__ const LinkWeights<Real<StepStore>> kLinkWeights = LinkWeights<Real<StepStore>>();
 
 template <class T>
 __device__ __forceinline__ void linkWeights(unsigned code, bool ibb, T& wPre, T& wPost, T& invDen) {
+    const T* w = kLinkWeights.v[code];
+    T t[3];
     if constexpr (sizeof(T) == 4) {
-        const float4 w = __ldg(reinterpret_cast<const float4*>(kLinkWeights.v[code]));
-        wPre = ibb ? w.x : 0.5f * (1.f / 1.5f);
-        wPost = ibb ? w.y : 0.5f * (1.f / 1.5f);
-        invDen = ibb ? w.z : 1.f / 1.5f;
+        const float4 q = __ldg(reinterpret_cast<const float4*>(w));
+        t[0] = q.x;
+        t[1] = q.y;
+        t[2] = q.z;
     } else {
-        const T q = static_cast<T>(code) / T(254);
-        const T gamma = !ibb ? T(0.5) : q < T(0.01f) ? T(0.01f) : q > T(1) ? T(1) : q;
-        invDen = T(1) / (T(1) + gamma);
-        wPre = (T(1) - gamma) * invDen;
-        wPost = gamma * invDen;
+        const double2 q = __ldg(reinterpret_cast<const double2*>(w));
+        t[0] = q.x;
+        t[1] = q.y;
+        t[2] = __ldg(w + 2);
     }
+    wPre = ibb ? t[0] : T(0.5) * (T(1) / T(1.5));
+    wPost = ibb ? t[1] : T(0.5) * (T(1) / T(1.5));
+    invDen = ibb ? t[2] : T(1) / T(1.5);
 }
 
 // Cells outside the bulk segments, one thread per listed cell: wall-adjacent
